@@ -177,14 +177,21 @@ def _prepare_fit(case, seed):
     return dict(case=case, train=pools[0], eval=pools[1], held=pools[2], params=params)
 
 
-def _stored_model(case, seed):
-    """A model as a service loads it from a file: random splits over a grid of borders, leaf values that shrink."""
+def _trees(case, seed):
+    """Random splits over a grid of borders, leaf values that shrink: (grid, split features, split borders, leaf values)."""
     rng = np.random.default_rng(int(seed))
     F, T, D, dims = case["cols"], case["trees"], case["depth"], case["dims"]
     grid = np.sort(rng.standard_normal((F, case["borders"])).astype(np.float32), axis=1)
     feat = rng.integers(0, F, (T, D))
     pick = rng.integers(0, case["borders"], (T, D))
     vals = rng.standard_normal((T, (1 << D) * dims)) * 0.1 / (1.0 + np.arange(T)[:, None] / 100.0)
+    return grid, feat, pick, vals
+
+
+def _stored_model(case, seed):
+    """A model as a service loads it from a file."""
+    F, T, D, dims = case["cols"], case["trees"], case["depth"], case["dims"]
+    grid, feat, pick, vals = _trees(case, seed)
     doc = {"features_info": {"float_features": [
         {"feature_index": j, "flat_feature_index": j, "borders": grid[j].tolist(), "has_nans": False,
          "nan_value_treatment": "AsIs", "feature_id": str(j)} for j in range(F)]},
@@ -197,12 +204,16 @@ def _stored_model(case, seed):
     return cb.CatBoost().load_model(blob=json.dumps(doc).encode(), format="json")
 
 
+def _rows(case, seed):
+    gen = torch.Generator(device="cuda").manual_seed(int(seed))
+    return torch.randn((case["rows"], case["cols"]), generator=gen, device="cuda")
+
+
 def prepare(case, seed):
     if case["kind"] == "fit":
         return _prepare_fit(case, seed)
-    gen = torch.Generator(device="cuda").manual_seed(int(seed))
     model = _stored_model(case, seed)
-    X = torch.randn((case["rows"], case["cols"]), generator=gen, device="cuda")
+    X = _rows(case, seed)
     if case["kind"] == "score":
         return dict(case=case, model=model, predictor=GpuPredictor(model._model), X=X)
     return dict(case=case, model=model, X=_host(X))
@@ -246,3 +257,22 @@ def tolerance(case):
     # code twice, and histograms summed in 13 to 16 against 24 bits a document): 53 pairs agree to 3e-5, two have one tree
     # that differs, which moves the predictions by 0.010 and 0.017 and leaves the loss curve alone to 1e-4.
     return {"rel": 0.03, "max": 0.9}
+
+
+def exact(case, seed):
+    """The sum of the leaves in 64 bits; a whole fit has no such value."""
+    if case["kind"] == "fit":
+        return None
+    grid, feat, pick, vals = _trees(case, seed)
+    columns = _rows(case, seed).t().contiguous()
+    vals = torch.from_numpy(vals).cuda().view(case["trees"], 1 << case["depth"], case["dims"])
+    out = torch.full((case["rows"], case["dims"]), 0.1, dtype=torch.float64, device="cuda")
+    for t in range(case["trees"]):
+        leaf = torch.zeros(case["rows"], dtype=torch.int64, device="cuda")
+        for d in range(case["depth"]):
+            j = int(feat[t, d])
+            leaf |= (columns[j] > float(grid[j, pick[t, d]])).long() << d
+        out += vals[t][leaf]
+    if case["kind"] == "score":
+        return out.t().contiguous()
+    return (out[:, 0] if case["dims"] == 1 else out).cpu().numpy()
