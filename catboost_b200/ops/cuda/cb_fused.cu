@@ -20,6 +20,7 @@
 #include "cb_common.cuh"
 #include <cstdlib>
 #include "cb_tree.cuh"
+#include "cb_lanes.cuh"
 #include "cb_comm.cuh"
 #include <cooperative_groups.h>
 #include <new>
@@ -116,7 +117,94 @@ static __device__ void cb_reduce_chunks(const CbFusedArgs& a, int cta, int ncta,
     }
 }
 
-__global__ void __launch_bounds__(1024, 1) cb_level_fused_kernel(CbFusedArgs a) {
+// The same for the feature-per-lane path, whose tiles are [slot][bin][NS][32 lanes].  A unit is four bins of one (slot,
+// statistic of the lane) row: a warp adds four 128-byte rows per chunk and every lane stores the 16 bytes of its feature.
+// With few units the chunks of a unit are dealt to KS warps of a block, which meet in shared memory.  Sums in 64 bits: with
+// up to 148 chunks an fp32 sum would be the largest error of a dense column's histogram.
+static __device__ void cb_reduce_lanes(const CbFusedArgs& a, float* sh, int cta, int ncta, unsigned int ll_tag) {
+    const CbHistArgs& h = a.h;
+    const int nslots = cb_hist_nslots(h);
+    const int R = a.c.nranks, me = a.c.rank;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    const CbBundle last = h.btab[h.nbundles - 1];
+    const int units = last.unit0 + nslots * (last.B >> 2) * (last.FL == 32 ? 2 : 1);
+    int KS = 1;
+    while (KS * 2 <= nwarp && (long long)units * (KS * 2) <= (long long)ncta * nwarp && KS * 2 <= h.nK) KS <<= 1;
+    const int upb = nwarp / KS, ks = warp % KS;
+    double4* red = reinterpret_cast<double4*>(sh);
+    for (int ub = cta * upb; ub < units; ub += ncta * upb) {
+        const int u = warp / KS < upb ? ub + warp / KS : units;
+        double4 sum = make_double4(0.0, 0.0, 0.0, 0.0);
+        CbBundle bd;
+        int slot = 0, b4 = 0, s = 0, NS = 1;
+        if (u < units) {
+            int lo = 0, hi = h.nbundles - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (h.btab[mid].unit0 <= u) lo = mid; else hi = mid - 1;
+            }
+            bd = h.btab[lo];
+            NS = bd.FL == 32 ? 2 : 1;
+            int v = u - bd.unit0;
+            s = v % NS; v /= NS;
+            b4 = v % (bd.B >> 2);
+            slot = v / (bd.B >> 2);
+            const int rs = NS * 32;
+            const size_t kstride = (size_t)nslots * bd.B * rs;
+            const float* src = h.priv + bd.priv0 + ((size_t)slot * bd.B + b4 * 4) * rs + s * 32 + lane;
+#pragma unroll 4
+            for (int k = ks; k < bd.nK; k += KS) {
+                const float* q = src + (size_t)k * kstride;
+                const float x = __ldcg(q), y = __ldcg(q + rs), z = __ldcg(q + 2 * rs), w = __ldcg(q + 3 * rs);
+                sum.x += x; sum.y += y; sum.z += z; sum.w += w;
+            }
+        }
+        if (KS > 1) {
+            red[threadIdx.x] = sum;
+            __syncthreads();
+            if (ks == 0)
+                for (int w = 1; w < KS; ++w) {
+                    const double4 t = red[(warp + w) * 32 + lane];
+                    sum.x += t.x; sum.y += t.y; sum.z += t.z; sum.w += t.w;
+                }
+            __syncthreads();
+        }
+        if (u >= units || ks != 0) continue;
+        float4 acc = make_float4((float)sum.x, (float)sum.y, (float)sum.z, (float)sum.w);
+        if (bd.FL == 8) {                              // two replicas, one per document of a reduction
+            acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 16);
+            acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 16);
+            acc.z += __shfl_xor_sync(0xffffffffu, acc.z, 16);
+            acc.w += __shfl_xor_sync(0xffffffffu, acc.w, 16);
+            if (lane >= 16) continue;
+        }
+        const int fl = lane & (bd.FL - 1);
+        const int f = bd.g0 * 4 + fl;
+        if (fl >= bd.gcnt * 4 || f >= h.d.F) continue;
+        const int col = h.d.feat_off[f] + b4 * 4;
+        if (col >= h.d.feat_off[f + 1]) continue;
+        const int row = slot * 2 + (NS == 2 ? s : lane / bd.FL);
+        if (R > 1) {
+            int r = 0;
+            while (r + 1 < R && col >= a.own_col[r + 1]) ++r;
+            unsigned long long* dst = reinterpret_cast<unsigned long long*>(a.c.peer_slot[r] + (size_t)me * a.c.slot_floats)
+                                      + (size_t)row * a.Wmax + (col - a.own_col[r]);
+            const unsigned long long t = (unsigned long long)ll_tag << 32;
+            const unsigned long long w0 = t | __float_as_uint(acc.x), w1 = t | __float_as_uint(acc.y);
+            const unsigned long long w2 = t | __float_as_uint(acc.z), w3 = t | __float_as_uint(acc.w);
+            asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(dst), "l"(w0), "l"(w1) : "memory");
+            asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(dst + 2), "l"(w2), "l"(w3) : "memory");
+        } else {
+            *reinterpret_cast<float4*>(const_cast<float*>(a.s.hsrc[0]) + (size_t)row * a.Wmax + col) = acc;
+        }
+    }
+    __syncthreads();
+}
+
+// LANES: the feature-per-lane histogram pass (two statistics, fixed point); a separate instantiation, so that neither
+// path's registers and instruction lines burden the other.
+template <bool LANES>
+__global__ void __launch_bounds__(LANES ? CB_LANE_THREADS : 1024, 1) cb_level_fused_kernel(CbFusedArgs a) {
     extern __shared__ __align__(16) float cb_sh[];
     cg::grid_group grid = cg::this_grid();
     const int cta = blockIdx.x, ncta = gridDim.x;
@@ -131,7 +219,7 @@ __global__ void __launch_bounds__(1024, 1) cb_level_fused_kernel(CbFusedArgs a) 
     const unsigned int ll_tag = (R > 1) ? cb_ll_tag(hist_epoch) : 0u;
 
     // (0) leaf update with the split of the previous level: its own pass, unless the histogram pass does it
-    if (level > 0 && !a.fuse_leaf) {
+    if (!LANES && level > 0 && !a.fuse_leaf) {
         cb_update_leaf_range(a.h.d, a.leaf, sp_arr[level - 1], level - 1,
                              (long long)cta * blockDim.x + threadIdx.x, (long long)ncta * blockDim.x);
         __threadfence();
@@ -143,7 +231,8 @@ __global__ void __launch_bounds__(1024, 1) cb_level_fused_kernel(CbFusedArgs a) 
     if (threadIdx.x == 0) s_noise_std = cb_noise_std(a.s);
     if (ts) ts[1] = cb_globaltimer();
     // (A) local histograms: every block dumps its shared-memory tile into its private region (no atomics)
-    cb_hist_phase(a.h, cb_sh, cta, ncta);
+    if (LANES) cb_lane_phase(a.h, reinterpret_cast<int*>(cb_sh), cta, ncta);
+    else cb_hist_phase(a.h, cb_sh, cta, ncta);
     if (ts) ts[2] = cb_globaltimer();
     if (a.phase_ts && threadIdx.x == 0 && level == a.depth - 2) {
         unsigned int smid;
@@ -158,7 +247,8 @@ __global__ void __launch_bounds__(1024, 1) cb_level_fused_kernel(CbFusedArgs a) 
     // (B) chunk reduction fused with the reduce-scatter: each 16-byte column group is summed over the chunks of
     // this rank and stored straight into the slot of the rank that owns the column (peer store over NVLink when
     // that is another GPU; every source keeps its own slot, so the owner later adds them in rank order).
-    cb_reduce_chunks(a, cta, ncta, ll_tag);
+    if (LANES) cb_reduce_lanes(a, cb_sh, cta, ncta, ll_tag);
+    else cb_reduce_chunks(a, cta, ncta, ll_tag);
     if (R <= 1) {
         __threadfence();
         grid.sync();
@@ -236,6 +326,15 @@ struct CbFusedPlan {
     int* d_gchunks[CB_MAX_LEVELS];     // document chunks of every feature group (those of its bundle)
     int n_btab[CB_MAX_LEVELS], n_items[CB_MAX_LEVELS];
     int single_pass_bundle[CB_MAX_LEVELS];     // 1: one bundle holds every group in one pass (leaf update can be fused)
+    // feature-per-lane path (cb_lanes.cuh)
+    const uint32_t* lanes;
+    const short* ldom;
+    cudaStream_t lane_stream;                  // the stream the lane store was made on; the work lists go there too
+    int lane_smem;                             // dynamic shared memory one block of that kernel may use
+    int lane_level[CB_MAX_LEVELS];             // 1: the level takes that path
+    long long lane_priv[CB_MAX_LEVELS];        // floats of its private tiles
+    long long lane_list[CB_MAX_LEVELS];        // entries of its document lists
+    unsigned int* d_cap[CB_MAX_LEVELS];
 };
 
 
@@ -281,15 +380,22 @@ CB_API CbFusedPlan* cb_fused_create(const CbData* d, const CbComm* comm, unsigne
     cudaDeviceGetAttribute(&p->max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     // dynamic shared memory available to this kernel = opt-in maximum minus its static shared memory
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, cb_level_fused_kernel) != cudaSuccess) { cudaGetLastError(); delete p; return nullptr; }
+    if (cudaFuncGetAttributes(&fa, cb_level_fused_kernel<false>) != cudaSuccess) { cudaGetLastError(); delete p; return nullptr; }
     p->max_smem -= (int)fa.sharedSizeBytes;
     cudaDeviceGetAttribute(&p->sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
     p->sm_smem -= 2 * (int)fa.sharedSizeBytes;
     p->max_bundle = 0;
+    p->lanes = nullptr; p->ldom = nullptr; p->lane_stream = nullptr;
+    cudaFuncAttributes fl;
+    if (cudaFuncGetAttributes(&fl, cb_level_fused_kernel<true>) != cudaSuccess) { cudaGetLastError(); delete p; return nullptr; }
+    p->lane_smem = p->max_smem + (int)fa.sharedSizeBytes - (int)fl.sharedSizeBytes;
+    for (int l = 0; l < CB_MAX_LEVELS; ++l) { p->lane_level[l] = 0; p->lane_priv[l] = 0; p->lane_list[l] = 0; p->d_cap[l] = nullptr; }
+    a.h.lanes = nullptr; a.h.ldom = nullptr; a.h.bcap = nullptr; a.h.list_q = nullptr; a.h.list_row = nullptr; a.h.nbundles = 0;
     for (int l = 0; l < CB_MAX_LEVELS; ++l) { p->d_btab[l] = nullptr; p->d_items[l] = nullptr; p->d_gchunks[l] = nullptr; p->n_btab[l] = p->n_items[l] = 0; p->single_pass_bundle[l] = 0; }
     p->max_copies = 2;
     p->fuse_leaf_update = 1;
-    if (cudaFuncSetAttribute(cb_level_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, p->max_smem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(cb_level_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, p->max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(cb_level_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, p->lane_smem) != cudaSuccess) {
         cudaGetLastError();
         delete p;
         return nullptr;
@@ -318,6 +424,7 @@ CB_API void cb_fused_destroy(CbFusedPlan* p) {
         if (p->d_btab[l]) cudaFree(p->d_btab[l]);
         if (p->d_items[l]) cudaFree(p->d_items[l]);
         if (p->d_gchunks[l]) cudaFree(p->d_gchunks[l]);
+        if (p->d_cap[l]) cudaFree(p->d_cap[l]);
     }
     delete p;
 }
@@ -334,12 +441,214 @@ CB_API void cb_fused_set_max_copies(CbFusedPlan* p, int max_copies) {
     p->max_copies = max_copies >= 8 ? 8 : (max_copies >= 4 ? 4 : (max_copies >= 2 ? 2 : 1));
 }
 
+// The lane-ordered copy of the store (words the caller allocates: cb_lane_store_words) and every feature's most frequent
+// bin, [4 G] on the device; call before cb_fused_geometry.
+CB_API long long cb_lane_store_words(long long n, int G) {
+    const long long npad = cb_lane_npad(n);
+    return (G >> 3) * 8 * npad + ((G & 7) ? cb_lane_row(G & 7, 0) * npad : 0);
+}
+CB_API int cb_lane_store(const CbData* d, uint32_t* lanes, cudaStream_t st) {
+    const long long total = (long long)((d->G + 7) >> 3) * (cb_lane_npad(d->n) >> 2) * 8;
+    const long long blocks = (total + 255) / 256;
+    if (blocks == 0) return 0;
+    cb_lane_store_kernel<<<(int)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, st>>>(*d, lanes);
+    return (int)cudaGetLastError();
+}
+CB_API void cb_fused_set_lanes(CbFusedPlan* p, const uint32_t* lanes, const short* ldom, cudaStream_t st) {
+    p->lanes = lanes;
+    p->ldom = ldom;
+    p->lane_stream = st;
+}
+// Floats of private tiles the level needs when it takes the feature-per-lane path (0: it does not).
+CB_API long long cb_fused_lane_priv(CbFusedPlan* p, int level) {
+    return level < CB_MAX_LEVELS && p->lane_level[level] ? p->lane_priv[level] : 0;
+}
+
+// Document list entries (12 bytes each) of the level, and their place.
+CB_API long long cb_fused_lane_list(CbFusedPlan* p, int level) {
+    return level < CB_MAX_LEVELS && p->lane_level[level] ? p->lane_list[level] : 0;
+}
+CB_API void cb_fused_set_lane_list(CbFusedPlan* p, int2* q, unsigned int* row) {
+    p->a.h.list_q = q;
+    p->a.h.list_row = row;
+}
+
+// Feature-per-lane geometry of one level: grid size, 0 = take the other path, -1 = error.
+static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass, int* smem_bytes, int* threads, int* chunks,
+                                  int* copies, int* bundle) {
+    const int nslots = level == 0 ? 1 : (1 << (level - 1));
+    const int G = p->a.h.d.G;
+    const long long n = p->a.h.d.n;
+    auto gb = [&](int g) { return p->group_bins.empty() ? p->a.h.B : p->group_bins[g]; };
+    const int ints = p->lane_smem / 4 - cb_lane_extra_ints(0);
+    // Cost of streaming 32 documents through a bundle: a fixed part per slot pass and a part per document taken.
+    const double taken = level == 0 ? 32.0 : 15.0;
+    auto shape = [&](int g, int gc, CbBundle* b) {
+        int B = 4;
+        for (int q = 0; q < gc; ++q) B = gb(g + q) > B ? gb(g + q) : B;
+        const int FL = gc > 4 ? 32 : (gc > 2 ? 16 : 8);
+        const int per = B * (FL == 32 ? 64 : 32) + 64;
+        int spp = ints / per;
+        if (spp < 1) return 1e30;
+        if (spp > 256) spp = 256;                      // eight bits of a staged entry
+        if (spp > nslots) spp = nslots;
+        const int np = (nslots + spp - 1) / spp;
+        spp = (nslots + np - 1) / np;
+        *b = CbBundle{g, gc, B, 1, spp, np, 1, FL, 0, 0, 0, 0, 0};
+        return np * 25.0 + taken * (FL == 32 ? 3.2 : (FL == 16 ? 2.2 : 1.2));
+    };
+    std::vector<CbBundle> bundles;
+    std::vector<double> cost;
+    for (int g = 0; g < G; g += 8) {
+        const int gc = G - g < 8 ? G - g : 8;
+        // a row block is one bundle, or is cut into halves (quarters) where a narrower tile saves enough slot passes
+        CbBundle w, h[2], t[4];
+        const double cw = shape(g, gc, &w);
+        std::vector<CbBundle> cut;
+        std::vector<double> ccut;
+        for (int half = 0; half < 2 && half * 4 < gc; ++half) {
+            const int hc = gc - half * 4 < 4 ? gc - half * 4 : 4;
+            const double ch = shape(g + half * 4, hc, &h[half]);
+            double cq = 1e30, c0 = 0.0, c1 = 0.0;
+            if (hc > 2) {
+                c0 = shape(g + half * 4, 2, &t[half * 2]);
+                c1 = shape(g + half * 4 + 2, hc - 2, &t[half * 2 + 1]);
+                cq = c0 + c1;
+            }
+            if (cq < ch) {
+                cut.push_back(t[half * 2]); ccut.push_back(c0);
+                cut.push_back(t[half * 2 + 1]); ccut.push_back(c1);
+            } else { cut.push_back(h[half]); ccut.push_back(ch); }
+        }
+        double sum = 0.0;
+        for (double c : ccut) sum += c;
+        if (cw <= sum) { bundles.push_back(w); cost.push_back(cw); }
+        else for (size_t i = 0; i < cut.size(); ++i) { bundles.push_back(cut[i]); cost.push_back(ccut[i]); }
+    }
+    for (double c : cost) if (c >= 1e29) return 0;
+    const int nbun = (int)bundles.size();
+    if (nbun < 1 || nbun > 0xFFFF) return 0;
+    int smem = 0;
+    for (const CbBundle& b : bundles) {
+        const int need = (b.spp * b.B * (b.FL == 32 ? 64 : 32) + cb_lane_extra_ints(b.spp)) * 4;
+        if (need > smem) smem = need;
+    }
+    const int want = 8 * CB_SCORE_WARP_FLOATS * 4;
+    if (smem < want) smem = want;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cb_level_fused_kernel<true>, CB_LANE_THREADS, smem) != cudaSuccess) { cudaGetLastError(); return -1; }
+    if (occ < 1) return 0;
+    const int grid = p->sm_count;                      // one block per SM
+    // chunks: every item about the same time, their number a whole multiple of the grid; no more chunks than steps of a
+    // thread block (and at most 4096, which keeps two strides inside 32 bits)
+    const long long nblk = (n + 2 * CB_LANE_THREADS - 1) / (2 * CB_LANE_THREADS);
+    const int most = (int)(nblk < 1 ? 1 : (nblk < 4096 ? nblk : 4096));
+    // The leaves of two slot passes hold different numbers of documents, so passes as items of their own leave blocks waiting
+    // (10.5M x 28, two passes in one round of items: blocks finished between 98 and 230 us).  An item takes its chunk
+    // through all passes where there are chunks enough for every SM; a small shard spreads its passes over the SMs instead.
+    const int seq = nblk >= grid && nslots <= 256 ? 1 : 0;         // (a list entry has eight bits for the slot)
+    double W = 0.0;
+    int min_items = 0;
+    bool mixed = false;
+    std::vector<int> per(nbun);                        // items a chunk of the bundle takes
+    for (int i = 0; i < nbun; ++i) {
+        bundles[i].seq = seq;
+        per[i] = seq ? 1 : bundles[i].npass;
+        W += cost[i];
+        min_items += per[i];
+        if (cost[i] != cost[0]) mixed = true;
+    }
+    const int rounds = (mixed && p->a.h.work) ? 2 : 1;      // items of different times are handed out by a counter
+    long long T = (long long)grid * rounds;
+    while (T < min_items) T += grid;
+    long long used = 0;
+    for (int i = 0; i < nbun; ++i) {
+        const double each = cost[i] / per[i];
+        int k = (int)((double)T * each / W);
+        k = k < 1 ? 1 : (k > most ? most : k);
+        bundles[i].nK = k;
+        used += (long long)k * per[i];
+    }
+    for (;;) {
+        int pick = -1;
+        double worst = 0.0;
+        for (int i = 0; i < nbun; ++i) {
+            if (used + per[i] > T || bundles[i].nK >= most) continue;
+            const double t = cost[i] / per[i] / bundles[i].nK;
+            if (t > worst) { worst = t; pick = i; }
+        }
+        if (pick < 0) break;
+        ++bundles[pick].nK;
+        used += per[pick];
+    }
+    int best = 1, unit = 0;
+    long long priv = 0, list = 0;
+    std::vector<unsigned int> cap(nbun);
+    for (int i = 0; i < nbun; ++i) {
+        CbBundle& b = bundles[i];
+        if (b.nK > best) best = b.nK;
+        const int NS = b.FL == 32 ? 2 : 1;
+        b.unit0 = unit;
+        b.priv0 = priv;
+        unit += nslots * (b.B >> 2) * NS;
+        priv += (long long)b.nK * nslots * b.B * NS * 32;
+        b.list_stride = (int)((nblk + b.nK - 1) / b.nK) * (2 * CB_LANE_THREADS);
+        b.list0 = list;
+        if (b.seq && b.npass > 1) list += (long long)b.nK * b.list_stride;
+        // documents one lane total can receive
+        cap[i] = (unsigned int)(((nblk + b.nK - 1) / b.nK) * (2 * CB_LANE_THREADS / 32) + 1);
+    }
+    std::vector<int2> items;
+    std::vector<int> order(nbun);
+    for (int i = 0; i < nbun; ++i) order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+        return cost[x] / per[x] / bundles[x].nK > cost[y] / per[y] / bundles[y].nK; });
+    items.reserve((size_t)used);
+    for (int k = 0; k < best; ++k)
+        for (int bi : order)
+            if (k < bundles[bi].nK)
+                for (int ps = 0; ps < per[bi]; ++ps) items.push_back(make_int2(bi | (ps << 16), k));
+    if (p->d_btab[level]) { cudaFree(p->d_btab[level]); p->d_btab[level] = nullptr; }
+    if (p->d_items[level]) { cudaFree(p->d_items[level]); p->d_items[level] = nullptr; }
+    if (p->d_cap[level]) { cudaFree(p->d_cap[level]); p->d_cap[level] = nullptr; }
+    if (cudaMalloc(&p->d_btab[level], bundles.size() * sizeof(CbBundle)) != cudaSuccess ||
+        cudaMalloc(&p->d_items[level], items.size() * sizeof(int2)) != cudaSuccess ||
+        cudaMalloc(&p->d_cap[level], (size_t)nbun * sizeof(unsigned int)) != cudaSuccess) { cudaGetLastError(); return -1; }
+    cudaStream_t st = p->lane_stream;
+    cudaMemcpyAsync(p->d_btab[level], bundles.data(), bundles.size() * sizeof(CbBundle), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(p->d_items[level], items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(p->d_cap[level], cap.data(), cap.size() * sizeof(unsigned int), cudaMemcpyHostToDevice, st);
+    cb_lane_cap_kernel<<<grid, CB_LANE_THREADS, 256 * 32 * 4, st>>>(p->a.h.d, p->lanes, p->ldom, p->d_btab[level],
+                                                                    p->d_items[level], (int)items.size(), p->d_cap[level]);
+    if (cudaGetLastError() != cudaSuccess) return -1;
+    p->n_btab[level] = nbun;
+    p->n_items[level] = (int)items.size();
+    p->lane_level[level] = 1;
+    p->lane_priv[level] = priv;
+    p->lane_list[level] = list;
+    *slots_per_pass = bundles[0].spp;
+    *smem_bytes = smem;
+    *threads = CB_LANE_THREADS;
+    *chunks = best;
+    *copies = 1;
+    *bundle = bundles[0].gcnt;
+    return grid;
+}
+
 CB_API int cb_fused_geometry(CbFusedPlan* p, int level, int* slots_per_pass, int* smem_bytes, int* threads, int* chunks,
                              int* copies, int* bundle) {
     const int nslots = level == 0 ? 1 : (1 << (level - 1));
     const bool narrow = p->a.h.statmax && p->a.h.S == 2 && p->a.h.narrow;
     const int G = p->a.h.d.G;
     const long long n = p->a.h.d.n;
+    if (level < CB_MAX_LEVELS) {
+        p->lane_level[level] = 0;
+        // document and row numbers of that path are 32 bits wide, two work strides beyond the last document included
+        if (p->lanes && narrow && n < (1ll << 28)) {
+            const int grid = cb_fused_lane_geometry(p, level, slots_per_pass, smem_bytes, threads, chunks, copies, bundle);
+            if (grid != 0) return grid > 0 ? grid : 0;
+        }
+    }
     int thr = p->threads, spp = nslots, C = 1, gpc = 0, smem = 0;
     std::vector<CbBundle> bundles;
     if (narrow && p->max_bundle > 0) {
@@ -431,7 +740,7 @@ CB_API int cb_fused_geometry(CbFusedPlan* p, int level, int* slots_per_pass, int
         if (smem < want) smem = want;
     }
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cb_level_fused_kernel, thr, smem) != cudaSuccess) { cudaGetLastError(); return 0; }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cb_level_fused_kernel<false>, thr, smem) != cudaSuccess) { cudaGetLastError(); return 0; }
     if (occ < 1) return 0;
     if (occ > 4) occ = 4;
     const int grid = occ * p->sm_count;
@@ -552,15 +861,20 @@ CB_API int cb_fused_launch(CbFusedPlan* p, int level, float* hprev, float* hcur,
     // document is streamed by exactly one block.  With several bundles each of them would have to fetch that word as
     // well, which costs more than the separate pass (measured at 10.5M x 28, level 5, 4 bundles: +86 us against 18 us).
     const bool table = bundle > 0 && level < CB_MAX_LEVELS && p->d_btab[level] != nullptr;
+    const bool lanes = level < CB_MAX_LEVELS && p->lane_level[level];
+    a.h.lanes = lanes ? p->lanes : nullptr; a.h.ldom = p->ldom; a.h.bcap = lanes ? p->d_cap[level] : nullptr;
+    a.h.nbundles = table ? p->n_btab[level] : 0;
     a.h.btab = table ? p->d_btab[level] : nullptr;
     a.h.bitems = table ? p->d_items[level] : nullptr;
     a.h.nbitems = table ? p->n_items[level] : 0;
     a.h.gchunks = table ? p->d_gchunks[level] : nullptr;
     const bool whole = table ? p->single_pass_bundle[level] != 0 : bundle >= a.h.d.G;
     a.fuse_leaf = (level > 0 && whole && a.h.statmax && a.h.S == 2 && a.h.narrow && p->fuse_leaf_update) ? 1 : 0;
+    if (lanes) a.fuse_leaf = 1;            // that path always reads the split column next to the leaf index
     a.h.prev_splits = a.fuse_leaf ? a.splits : nullptr;
     void* args[] = {&a};
-    cudaError_t e = cudaLaunchCooperativeKernel((void*)cb_level_fused_kernel, dim3(grid), dim3(threads), args,
+    void* kernel = lanes ? (void*)cb_level_fused_kernel<true> : (void*)cb_level_fused_kernel<false>;
+    cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args,
                                                 (size_t)smem_bytes, st);
     return (int)e;
 }

@@ -43,6 +43,14 @@ struct CbBundle {
     int spp;           // slots (leaves) per pass
     int npass;
     int nK;            // document chunks of this bundle
+    // feature-per-lane path (cb_lanes.cuh): lanes a document takes (32, 16 or 8 features), the first of the bundle's units
+    // in the reduction over the chunks, and where its tiles start in the private region (floats)
+    int FL;
+    int unit0;
+    long long priv0;
+    int seq;           // 1: a work item takes its chunk through all slot passes, 0: every pass is an item of its own
+    int list_stride;   // seq: documents of a chunk at most, and where the bundle's lists start
+    long long list0;
 };
 
 struct CbHistArgs {
@@ -98,6 +106,14 @@ struct CbHistArgs {
     const int2* bitems;         // x = bundle | pass << 16, y = document chunk
     int nbitems;
     const int* gchunks;         // [G] document chunks of the bundle every group belongs to
+    // Feature-per-lane path: the lane-ordered copy of the store, every feature's most frequent bin and, per bundle, the
+    // most documents one cell can receive (cb_lanes.cuh).  nullptr = off.
+    const uint32_t* lanes;
+    const short* ldom;
+    const unsigned int* bcap;
+    int2* list_q;               // scratch: documents that the later slot passes of a work item take
+    unsigned int* list_row;
+    int nbundles;
     const CbSplit* prev_splits;
     const int* prev_iter;
     int prev_depth;

@@ -238,6 +238,12 @@ _SIGS = {
                                    c_float, c_void_p, c_void_p, c_ull, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int]),
     "cb_fused_set_fuse_leaf": (None, [c_void_p, c_int]),
     "cb_fused_set_dominant": (None, [c_void_p, c_void_p]),
+    "cb_lane_store_words": (c_ll, [c_ll, c_int]),
+    "cb_lane_store": (c_int, [c_void_p, c_void_p, c_void_p]),
+    "cb_fused_set_lanes": (None, [c_void_p, c_void_p, c_void_p, c_void_p]),
+    "cb_fused_lane_priv": (c_ll, [c_void_p, c_int]),
+    "cb_fused_lane_list": (c_ll, [c_void_p, c_int]),
+    "cb_fused_set_lane_list": (None, [c_void_p, c_void_p, c_void_p]),
     "cb_fused_set_features": (None, [c_void_p, c_int, c_int]),
     "cb_fused_set_phase_ts": (None, [c_void_p, c_void_p]),
     "cb_fused_set_work": (None, [c_void_p, c_void_p]),

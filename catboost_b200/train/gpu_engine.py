@@ -58,7 +58,8 @@ class GpuObliviousEngine:
                  timeout_s: float = 20.0, quantized_hist: bool = True, dynamic_work: bool = True,
                  der_fn=None, zero_mean_leaves: bool = False, max_bundle: int = 8,
                  fused_leaf_steps: bool = True, mvs_reg=None, leaf_backtracking: str = "AnyImprovement",
-                 fuse_leaf_update: bool = True, dims: int = 1, skip_dominant_bin: bool = True):
+                 fuse_leaf_update: bool = True, dims: int = 1, skip_dominant_bin: bool = True,
+                 lane_hist: bool = False):
         assert store.bins.is_cuda, "GpuObliviousEngine needs a CUDA store"
         if depth > 16:
             raise ValueError("depth must be <= 16")
@@ -148,6 +149,7 @@ class GpuObliviousEngine:
         self.fuse_leaf_update = bool(fuse_leaf_update)
         self._check_each = os.environ.get("CB200_CHECK") == "1"      # invariants after every iteration (slow, debugging)
         self.skip_dominant_bin = bool(skip_dominant_bin) and os.environ.get("CB200_SKIP_DOMINANT", "1") != "0"
+        self.lane_hist = bool(lane_hist) and self.narrow_hist and self.S == 2 and store.F > 0
         self.stats = torch.zeros((self.S, npad), dtype=f32, device=dev)
         self.scal = torch.zeros(4, dtype=f64, device=dev)
         self.iter_ptr = torch.zeros(1, dtype=i32, device=dev)
@@ -266,6 +268,13 @@ class GpuObliviousEngine:
             self.domw = None
             if self.dominant_bin_share > gate:
                 self.lib.cb_fused_set_max_copies(ctypes.c_void_p(self.plan), 8)
+        if self.lane_hist:
+            # the feature-per-lane histogram pass reads its own copy of the store: a document's 32 features side by side
+            words = int(self.lib.cb_lane_store_words(self.n, self.store.G))
+            self.lane_store = torch.empty(max(words, 1), dtype=torch.int32, device=self.dev)
+            native.cuda_check(self.lib.cb_lane_store(ctypes.c_void_p(self.store.handle), _p(self.lane_store), self._stream()),
+                              "cb_lane_store")
+            self.lib.cb_fused_set_lanes(ctypes.c_void_p(self.plan), _p(self.lane_store), _p(self.top_bins), self._stream())
         self.work = torch.zeros(self.store.G + 1, dtype=torch.int32, device=self.dev)
         if self.dynamic_work:
             self.lib.cb_fused_set_work(ctypes.c_void_p(self.plan), _p(self.work))
@@ -282,8 +291,14 @@ class GpuObliviousEngine:
         need = 0
         for level, geo in enumerate(self.level_geo):
             nslots = 1 if level == 0 else 1 << (level - 1)
-            need = max(need, G * geo[4] * nslots * self.S * 4 * self.B)
+            lane = int(self.lib.cb_fused_lane_priv(ctypes.c_void_p(self.plan), level))
+            need = max(need, lane or G * geo[4] * nslots * self.S * 4 * self.B)
         self.priv = torch.empty(need, dtype=torch.float32, device=self.dev)
+        entries = max((int(self.lib.cb_fused_lane_list(ctypes.c_void_p(self.plan), l)) for l in range(self.depth)), default=0)
+        if entries:
+            self.lane_list = (torch.empty((entries, 2), dtype=torch.int32, device=self.dev),
+                              torch.empty(entries, dtype=torch.int32, device=self.dev))
+            self.lib.cb_fused_set_lane_list(ctypes.c_void_p(self.plan), _p(self.lane_list[0]), _p(self.lane_list[1]))
         self.lib.cb_fused_set_priv(ctypes.c_void_p(self.plan), _p(self.priv),
                                    _p(self.statmax) if self.quantized_hist else None)
 
@@ -343,9 +358,12 @@ class GpuObliviousEngine:
         decision.  A feature gets a dominant bin when at least 30 % of the sampled documents share one bin; the packed
         word of a group holds 255 for its other features."""
         st = self.store
+        G = st.bins.shape[0]
+        # every feature's most frequent bin (the feature-per-lane pass restores it from totals); -1 = padding column
+        self.top_bins = torch.full((G * 4,), -1, dtype=torch.int16, device=self.dev)
+        self.top_bins[: st.F] = 0
         if st.n <= 0 or st.F <= 0:
             return 0.0, None
-        G = st.bins.shape[0]
         step = max(1, st.n // sample)
         rows = st.bins[:, : st.n: step].contiguous()
         m = rows.shape[1]
@@ -357,6 +375,7 @@ class GpuObliviousEngine:
             self.ctx.all_reduce_sum_(cnt)
             self.ctx.all_reduce_sum_(tot)
         top, arg = cnt.max(1)
+        self.top_bins[: st.F] = arg[: st.F].to(torch.int16)
         share = top / tot.clamp_min(1.0)
         mean_share = float(share[: st.F].mean().item())
         dom = torch.where(share >= 0.30, arg, torch.full_like(arg, 255))

@@ -1,0 +1,103 @@
+"""The feature-per-lane histogram pass against sums in 64 bits, at the sizes where its row blocks, lane widths, slot passes
+and document blocks end."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _store(n, widths, seed, sparse=False):
+    """A binned store with one column per entry of ``widths`` (number of bins); bins drawn, not quantised."""
+    from catboost_b200.data.quantization import FlatFeature, make_store, pack_columns_into
+    rng = np.random.default_rng(seed)
+    feats = [FlatFeature("float", j, borders=np.arange(w - 1, dtype=np.float32), n_bins=w) for j, w in enumerate(widths)]
+    store = make_store(feats, n, torch.device("cuda"))
+    cols = np.stack([rng.integers(0, w, n) for w in widths]).astype(np.uint8)
+    if sparse:
+        cols[rng.random(cols.shape) < 0.7] = 0
+    pack_columns_into(store, torch.from_numpy(cols).cuda(), 0)
+    return store, cols
+
+
+def _engine(store, y, depth, lane_hist, **kw):
+    from catboost_b200.train.gpu_engine import GpuObliviousEngine
+    from catboost_b200.train.objectives import make_objective
+    args = dict(depth=depth, iterations=2, learning_rate=0.5, l2_leaf_reg=3.0, random_strength=0.0, bootstrap_type="Bayesian",
+                leaf_iterations=1, seed=3, lane_hist=lane_hist)
+    args.update(kw)
+    return GpuObliviousEngine(store, torch.from_numpy(y), None, torch.zeros(len(y)), make_objective("RMSE", {}), **args)
+
+
+@pytest.mark.parametrize("n,widths,depth,sparse", [
+    (1, [5], 1, False),
+    (255, [2, 3, 200], 3, False),
+    (1023, [17] * 8, 4, False),                      # one row block of two groups: 16 documents a load
+    (1025, [129] * 9, 6, False),                     # three groups: 8 documents a load
+    (30_011, [129] * 28, 6, False),                  # seven groups: 4 documents a load, several slot passes
+    (30_011, [129] * 28, 6, True),
+    (260_003, [129] * 28, 6, False),                 # chunks for every SM: the later passes read the first one's list
+    (5_000, [256] * 18, 6, False),                   # the widest columns, a row block of five groups
+    (20_007, [255] * 33 + [2] * 6, 7, False),        # a second row block of two groups
+    (9_999, [129] * 13 + [16] * 25 + [2] * 40, 8, True),     # narrow columns next to wide ones
+])
+def test_lane_histograms_equal_sums_in_64_bits(n, widths, depth, sparse):
+    store, cols = _store(n, widths, seed=n + len(widths), sparse=sparse)
+    rng = np.random.default_rng(n)
+    y = (cols[0] / widths[0] + 0.3 * rng.standard_normal(n) + (cols[-1] > 0)).astype(np.float32)
+    eng = _engine(store, y, depth, True)
+    eng.step(1)
+    torch.cuda.synchronize()
+    level = depth - 1
+    nslots = 1 if level == 0 else 1 << (level - 1)
+    W = eng.Wmax
+    got = eng.slots[: nslots * 2 * W].view(nslots, 2, W).cpu().numpy().astype(np.float64)
+    stats = eng.stats[:, :n].cpu().numpy().astype(np.float64)
+    leaf = eng.leaf[:n].cpu().numpy().astype(np.int64) & 0xFFFF
+    # leaf indices hold every split of the tree; those of the levels before this one decide the slot and the child
+    sp = eng.splits[:depth].cpu().numpy()
+    for d in range(depth):
+        bit = (cols[sp[d, 0]] > sp[d, 1]) if sp[d, 0] >= 0 else np.zeros(n, dtype=bool)
+        assert np.array_equal((leaf >> d) & 1, bit.astype(np.int64)), d
+    take, slot = np.ones(n, dtype=bool), np.zeros(n, dtype=np.int64)
+    if level > 0:
+        slot = leaf & (nslots - 1)
+        mask = eng.mask[level & 1].cpu().numpy().view(np.uint32)
+        want = (mask[slot >> 5] >> (slot & 31).astype(np.uint32)) & 1
+        take = ((leaf >> (level - 1)) & 1) == want
+    # a value is rounded to half a quantum; a cell holds at most n documents, so the quantum is at most
+    # max / (2^31 / n - 2), or max / 8388600 when that is coarser
+    smax = np.abs(stats).max(1)
+    quantum = smax / np.minimum(8388600.0, 2.0 ** 31 / (n + 2) - 2.0)
+    off = store.feat_off_host
+    for f, w in enumerate(widths):
+        for s in range(2):
+            oracle = np.zeros((nslots, w))
+            count = np.zeros((nslots, w))
+            mass = np.zeros((nslots, w))
+            np.add.at(oracle, (slot[take], cols[f][take]), stats[s][take])
+            np.add.at(count, (slot[take], cols[f][take]), 1.0)
+            np.add.at(mass, (slot[take], cols[f][take]), np.abs(stats[s][take]))
+            err = np.abs(got[:, s, off[f]: off[f] + w] - oracle)
+            # rounding of the documents, of the scale (24 bits), and of the fp32 sums over the chunks
+            tol = 0.5 * quantum[s] * count + mass * 2.0 ** -20 + 1e-30
+            assert (err <= tol).all(), (f, s, float((err / tol).max()))
+    eng.finish()
+    eng.close()
+
+
+@pytest.mark.parametrize("n,F,borders,depth", [(40_001, 30, 128, 6), (3_000, 12, 128, 6), (60_013, 39, 254, 8)])
+def test_lane_pass_grows_the_trees_of_the_other_pass(n, F, borders, depth):
+    store, cols = _store(n, [borders + 1] * F, seed=F)
+    rng = np.random.default_rng(1)
+    y = (np.sin(cols[0] / 20.0) + (cols[1] > 60) * (cols[2] > 40) + 0.01 * cols[5] + 0.2 * rng.standard_normal(n)).astype(np.float32)
+    outs = []
+    for lanes in (True, False):
+        eng = _engine(store, y, depth, lanes, iterations=3, leaf_iterations=2)
+        eng.step(3)
+        outs.append([a.copy() for a in eng.finish()] + [eng.learn_loss_history()])
+        eng.close()
+    # the first tree sees the same statistics; a later level of it may meet two candidates equal to within the quantum
+    same = (outs[0][0][0, :, :2] == outs[1][0][0, :, :2]).all(-1)
+    assert same[: min(depth, 5)].all(), (outs[0][0][0], outs[1][0][0])
+    assert np.allclose(outs[0][3], outs[1][3], rtol=5e-3)
