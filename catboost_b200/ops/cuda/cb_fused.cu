@@ -533,7 +533,8 @@ static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass
         const int need = (b.spp * b.B * (b.FL == 32 ? 64 : 32) + cb_lane_extra_ints(b.spp)) * 4;
         if (need > smem) smem = need;
     }
-    const int want = 8 * CB_SCORE_WARP_FLOATS * 4;
+    // the score phase reuses the tile as scratch; one block per SM runs either way, so every warp gets some
+    const int want = (CB_LANE_THREADS / 32) * CB_SCORE_WARP_FLOATS * 4;
     if (smem < want) smem = want;
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cb_level_fused_kernel<true>, CB_LANE_THREADS, smem) != cudaSuccess) { cudaGetLastError(); return -1; }

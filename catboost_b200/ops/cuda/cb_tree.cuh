@@ -975,12 +975,6 @@ __device__ __forceinline__ unsigned int cb_score_tag(const CbScoreArgs& a) {
     return a.ll_epoch ? cb_ll_tag(*a.ll_epoch + 1ull) : 0u;
 }
 
-__device__ __forceinline__ float cb_score_src(const CbScoreArgs& a, int r, size_t idx, unsigned int tag) {
-    if (tag == 0u) return __ldcg(a.hsrc[r] + idx);
-    const unsigned long long* w = reinterpret_cast<const unsigned long long*>(a.hsrc[r]) + idx;
-    return __uint_as_float(cb_ll_load(w, tag, a.ll_timeout_ns, a.ll_status, CB_TIMEOUT_HIST_ARRIVE, r));
-}
-
 __device__ __forceinline__ void cb_score_add_leaf(int fn, float l2, float s, float w, float& num, float& den) {
     switch (fn) {
         default:
@@ -1019,50 +1013,33 @@ __device__ __forceinline__ float cb_noise_std(const CbScoreArgs& a) {
     return (float)(a.random_strength * sd * (m / (1.0 + m)));
 }
 
-// Scoring is written as short rolled loops over 32-bin chunks with its accumulators in shared memory: a level runs
-// this code once, on a handful of warps, straight after a phase that evicted it from the instruction caches, so its
-// run time is the number of instruction lines it has to fetch, not the arithmetic.
-// Per-warp scratch (floats): num[256], den[256], pw[256] (prefix of the weight column), ps[256] (prefix of a
-// derivative column).
-#define CB_SCORE_WARP_FLOATS 1024
+// A warp scores the two children of one parent together: the histogram of the accumulated child and the parent's are
+// loaded once, every load of the pair before the first use, and the sibling is their difference -- what a warp waits for
+// is one trip to L2 per pair instead of four (60K x 39, 254 borders, level 7: 95 us with a trip per leaf and statistic).
+// The loops over the bins of a lane are rolled and keep their arrays in shared memory: a level runs this code once, on a
+// handful of warps, straight after a phase that evicted it from the instruction caches, so long unrolled code waits for
+// its own instruction lines.
+// Per-warp scratch (floats): num[256], den[256], then the in-lane prefixes of the two children, weight and derivative.
+// Lane l owns bins l * V .. l * V + V - 1, V = ceil(bins / 32); its k-th bin is at k * 32 + l of every array.
+#define CB_SCORE_WARP_FLOATS 1536
 
-// Column `st` of leaf l for the 32 bins of chunk c: summed over the sources, completed from the parent when the leaf
-// is the sibling that was not accumulated, stored into the complete histogram of this level.
-__device__ __forceinline__ float cb_score_load(const CbScoreArgs& a, int l, int p, bool computed, int st, int col0,
-                                               int bin, int nb, unsigned int tag) {
-    float x = 0.0f;
-    if (bin < nb) {
-        const size_t idx = ((size_t)p * a.S + st) * a.W + col0 + bin;
-        for (int r = 0; r < a.nsrc; ++r) x += cb_score_src(a, r, idx, tag);
-        if (!computed) x = a.hprev[idx] - x;
-        if (a.hcur) a.hcur[((size_t)l * a.S + st) * a.W + col0 + bin] = x;
-    }
-    return x;
-}
-
-// The same for the up to 8 bins a lane owns (bins lane * bpl + k), with every load issued before the first use.  Used
-// when a warp walks many leaves of one feature: there the chain of dependent L2 round trips is what the warp waits for,
-// and the longer code is fetched once and reused for every leaf.
-__device__ __forceinline__ void cb_score_load8(const CbScoreArgs& a, int l, int p, bool computed, int st, int col0,
-                                               int lane, int bpl, int nb, float* x, unsigned int tag) {
-    const size_t base = ((size_t)p * a.S + st) * a.W + col0 + lane * bpl;
-    const int left = nb - lane * bpl;                  // bins of this lane that exist
-    float prev[8];
+// Bins lane * V + k of one column of a parent: x = the accumulated child, summed over the sources, prev = the parent.
+__device__ __forceinline__ void cb_score_load8(const CbScoreArgs& a, int p, int st, int col0, int lane, int V, int nb,
+                                               unsigned int tag, float (&x)[8], float (&prev)[8]) {
+    const size_t base = ((size_t)p * a.S + st) * a.W + col0 + lane * V;
+    const int left = nb - lane * V;                    // bins of this lane that exist
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { x[k] = 0.0f; prev[k] = 0.0f; }
     if (tag != 0u) {
         // tagged words: peek at all of a source's words first (the loads overlap), then poll the ones not there yet
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            x[k] = 0.0f;
-            prev[k] = (k < bpl && k < left && !computed) ? a.hprev[base + k] : 0.0f;
-        }
         for (int r = 0; r < a.nsrc; ++r) {
             const unsigned long long* w = reinterpret_cast<const unsigned long long*>(a.hsrc[r]) + base;
             unsigned long long v[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = (k < bpl && k < left) ? cb_ll_peek(w + k) : 0ull;
+            for (int k = 0; k < 8; ++k) v[k] = (k < V && k < left) ? cb_ll_peek(w + k) : 0ull;
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                if (k < bpl && k < left) {
+                if (k < V && k < left) {
                     unsigned int pay = (unsigned int)v[k];
                     if ((unsigned int)(v[k] >> 32) != tag)
                         pay = cb_ll_load(w + k, tag, a.ll_timeout_ns, a.ll_status, CB_TIMEOUT_HIST_ARRIVE, r);
@@ -1070,125 +1047,164 @@ __device__ __forceinline__ void cb_score_load8(const CbScoreArgs& a, int l, int 
                 }
             }
         }
-    } else {
+    }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const bool ok = k < bpl && k < left;
-            x[k] = ok ? __ldcg(a.hsrc[0] + base + k) : 0.0f;
-            prev[k] = (ok && !computed) ? a.hprev[base + k] : 0.0f;
+    for (int k = 0; k < 8; ++k) {
+        if (k < V && k < left) {
+            if (a.level > 0) prev[k] = __ldcg(a.hprev + base + k);
+            if (tag == 0u) x[k] = __ldcg(a.hsrc[0] + base + k);
         }
+    }
+    if (tag == 0u) {
         for (int r = 1; r < a.nsrc; ++r) {
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-                if (k < bpl && k < left) x[k] += __ldcg(a.hsrc[r] + base + k);
-        }
-    }
-    const size_t obase = ((size_t)l * a.S + st) * a.W + col0 + lane * bpl;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        if (k < bpl && k < left) {
-            if (!computed) x[k] = prev[k] - x[k];
-            if (a.hcur) a.hcur[obase + k] = x[k];
+                if (k < V && k < left) x[k] += __ldcg(a.hsrc[r] + base + k);
         }
     }
 }
 
-// Score terms of feature f accumulated over the leaves l0, l0 + lstep, ... into sc[0..255] (num) and sc[256..511]
-// (den); sc[512..] is scratch.  One warp.
-static __device__ void cb_score_accumulate(const CbScoreArgs& a, int f, int l0, int lstep, float* sc) {
+// In-lane prefixes of the values (one-hot: the values themselves) into pre, the sum of the lanes before this one and of all.
+__device__ __forceinline__ void cb_score_scan(const float (&v)[8], int lane, int V, bool onehot, float* pre, float& excl, float& total) {
+    float run = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (k < V) {
+            run += v[k];
+            pre[k * 32 + lane] = onehot ? v[k] : run;
+        }
+    }
+    float inc = run;
+    for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    excl = onehot ? 0.0f : inc - run;
+    total = __shfl_sync(0xffffffffu, inc, 31);
+}
+
+__device__ __forceinline__ void cb_score_store8(const CbScoreArgs& a, int l, int st, int col0, int lane, int V, int nb, const float (&v)[8]) {
+    float* out = a.hcur + ((size_t)l * a.S + st) * a.W + col0 + lane * V;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (k < V && lane * V + k < nb) out[k] = v[k];
+}
+
+__device__ __forceinline__ void cb_score_add_cosine(float l2, float s, float w, float& num, float& den) {
+    const float mu = (w > 0.0f) ? __fdividef(s, w + l2) : 0.0f;
+    num += s * mu;
+    den += w * mu * mu;
+}
+
+// Score terms of feature f accumulated over the parents p0, p0 + pstep, ... into sc[0..255] (num) and sc[256..511] (den).
+// One warp.
+static __device__ void cb_score_accumulate(const CbScoreArgs& a, int f, int p0, int pstep, float* sc) {
     const int lane = threadIdx.x & 31;
     const int nb = a.d.feat_nb[f];
     const int col0 = a.d.feat_off[f] - a.col_base;
     const bool onehot = a.d.feat_onehot && a.d.feat_onehot[f];
     const int S = a.S;
-    const int L = 1 << a.level;
-    const int half = L >> 1;
-    const int bpl = (nb + 31) >> 5;
+    const int V = (nb + 31) >> 5;
+    const int parents = a.level > 0 ? 1 << (a.level - 1) : 1;
+    const int kids = a.level > 0 ? 2 : 1;
     const unsigned int tag = cb_score_tag(a);
-    float* num = sc;
-    float* den = sc + 256;
-    float* pw = sc + 512;
-    float* ps = sc + 768;
-    for (int b = lane; b < 512; b += 32) sc[b] = 0.0f;
-    __syncwarp();
-    const bool batched = (L / lstep) >= 4 && bpl <= 8;       // several leaves per warp: overlap the loads of a leaf
-    for (int l = l0; l < L; l += lstep) {
-        int p = 0;
-        bool computed = true;
-        if (a.level > 0) {
-            p = l & (half - 1);
-            const unsigned int right = (unsigned int)l >> (a.level - 1);
-            computed = (((a.small_mask[p >> 5] >> (p & 31)) & 1u) == right);
-        }
-        float totw = 0.0f, exw = 0.0f;
-        for (int pass = 0; pass < S; ++pass) {           // weight column first, then the derivative columns
-            const bool is_w = pass == 0;
-            const int c_st = is_w ? S - 1 : pass - 1;
-            float* pre = is_w ? pw : ps;
-            // lane owns bins [lane * bpl, lane * bpl + bpl): inclusive prefix inside the lane, then one warp scan.
-            // (Issuing all loads of the leaf first in an unrolled loop was measured slower: more instruction lines to
-            // fetch cost more than the overlapped load latency saved.)
-            float run = 0.0f;
-            if (batched) {
-                float x8[8];
-                cb_score_load8(a, l, p, computed, c_st, col0, lane, bpl, nb, x8, tag);
+    float* num = sc + lane;
+    float* den = sc + 256 + lane;
+    float* pre = sc + 512;                             // [child][weight, derivative][256]
+    for (int k = 0; k < V; ++k) { num[k * 32] = 0.0f; den[k * 32] = 0.0f; }
+    for (int p = p0; p < parents; p += pstep) {
+        const unsigned int right = a.level > 0 ? (a.small_mask[p >> 5] >> (p & 31)) & 1u : 0u;
+        const int l0 = a.level > 0 ? p | (int)(right << (a.level - 1)) : 0;            // the accumulated child
+        const int l1 = a.level > 0 ? p | (int)((right ^ 1u) << (a.level - 1)) : 0;     // its sibling
+        float x[8], prev[8], xs[8], prevs[8];
+        cb_score_load8(a, p, S - 1, col0, lane, V, nb, tag, x, prev);                  // weights
+        cb_score_load8(a, p, 0, col0, lane, V, nb, tag, xs, prevs);
+        float exw0, exw1 = 0.f, tw0, tw1 = 0.f, ex0, ex1 = 0.f, t0, t1 = 0.f;
+        cb_score_scan(x, lane, V, onehot, pre, exw0, tw0);
+        if (a.hcur) cb_score_store8(a, l0, S - 1, col0, lane, V, nb, x);
+        if (kids == 2) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    if (k < bpl) {
-                        run += x8[k];
-                        pre[lane * bpl + k] = onehot ? x8[k] : run;
+            for (int k = 0; k < 8; ++k) x[k] = prev[k] - x[k];
+            cb_score_scan(x, lane, V, onehot, pre + 512, exw1, tw1);
+            if (a.hcur) cb_score_store8(a, l1, S - 1, col0, lane, V, nb, x);
+        }
+        for (int st = 0; st < S - 1; ++st) {
+            if (st > 0) cb_score_load8(a, p, st, col0, lane, V, nb, tag, xs, prevs);
+            cb_score_scan(xs, lane, V, onehot, pre + 256, ex0, t0);
+            if (a.hcur) cb_score_store8(a, l0, st, col0, lane, V, nb, xs);
+            if (kids == 2) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) xs[k] = prevs[k] - xs[k];
+                cb_score_scan(xs, lane, V, onehot, pre + 768, ex1, t1);
+                if (a.hcur) cb_score_store8(a, l1, st, col0, lane, V, nb, xs);
+            }
+            if (a.score_fn == CB_SCORE_COSINE) {
+#pragma unroll 1
+                for (int k = 0; k < V; ++k) {
+                    const float* q = pre + k * 32 + lane;
+                    float n_ = num[k * 32], d_ = den[k * 32];
+                    const float w0 = exw0 + q[0], s0 = ex0 + q[256];
+                    cb_score_add_cosine(a.l2, s0, fmaxf(w0, 0.0f), n_, d_);
+                    cb_score_add_cosine(a.l2, t0 - s0, fmaxf(tw0 - w0, 0.0f), n_, d_);
+                    if (kids == 2) {
+                        const float w1 = exw1 + q[512], s1 = ex1 + q[768];
+                        cb_score_add_cosine(a.l2, s1, fmaxf(w1, 0.0f), n_, d_);
+                        cb_score_add_cosine(a.l2, t1 - s1, fmaxf(tw1 - w1, 0.0f), n_, d_);
                     }
+                    num[k * 32] = n_;
+                    den[k * 32] = d_;
                 }
-            } else {
-                for (int k = 0; k < bpl; ++k) {
-                    const int bin = lane * bpl + k;
-                    const float x = cb_score_load(a, l, p, computed, c_st, col0, bin, nb, tag);
-                    run += x;
-                    pre[bin] = onehot ? x : run;
+                continue;
+            }
+#pragma unroll 1
+            for (int k = 0; k < V; ++k) {
+                float n_ = num[k * 32], d_ = den[k * 32];
+#pragma unroll 1
+                for (int c = 0; c < kids; ++c) {
+                    const float* q = pre + c * 512 + k * 32 + lane;
+                    const float tw = c ? tw1 : tw0, t = c ? t1 : t0;
+                    const float wlk = (c ? exw1 : exw0) + q[0], slk = (c ? ex1 : ex0) + q[256];
+                    cb_score_add_leaf(a.score_fn, a.l2, slk, fmaxf(wlk, 0.0f), n_, d_);
+                    cb_score_add_leaf(a.score_fn, a.l2, t - slk, fmaxf(tw - wlk, 0.0f), n_, d_);
                 }
-            }
-            float inc = run;
-            for (int o = 1; o < 32; o <<= 1) {
-                const float t = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += t;
-            }
-            const float excl = onehot ? 0.0f : inc - run;
-            const float total = __shfl_sync(0xffffffffu, inc, 31);
-            if (is_w) { totw = total; exw = excl; continue; }
-            for (int k = 0; k < bpl; ++k) {
-                const int bin = lane * bpl + k;
-                const float slk = excl + ps[bin], wlk = exw + pw[bin];
-                float n_ = num[bin], d_ = den[bin];
-                cb_score_add_leaf(a.score_fn, a.l2, slk, fmaxf(wlk, 0.0f), n_, d_);
-                cb_score_add_leaf(a.score_fn, a.l2, total - slk, fmaxf(totw - wlk, 0.0f), n_, d_);
-                num[bin] = n_; den[bin] = d_;
+                num[k * 32] = n_;
+                den[k * 32] = d_;
             }
         }
     }
 }
 
-// Best candidate of feature f from complete num/den (one warp); borders are bins 0 .. nb-2 (one-hot: every value).
-static __device__ void cb_score_finalize(const CbScoreArgs& a, int f, const float* num, const float* den, float noise_std) {
+// Best candidate of feature f from the num / den of its `parts` warps (CB_SCORE_WARP_FLOATS apart); this warp takes every
+// pstep-th row of 32 bins.  Borders are bins 0 .. nb-2 (one-hot: every value).
+static __device__ void cb_score_finalize(const CbScoreArgs& a, int f, const float* sc, int parts, int k0, float noise_std) {
     const int lane = threadIdx.x & 31;
     const int nb = a.d.feat_nb[f];
+    const int V = (nb + 31) >> 5;
     const float fw = a.d.feat_weight ? a.d.feat_weight[f] : 1.0f;
     const bool onehot = a.d.feat_onehot && a.d.feat_onehot[f];
     unsigned long long best = 0ull;
     if (fw > 0.0f) {
         const int ncand = onehot ? nb : nb - 1;
         const unsigned long long it = (unsigned long long)(*a.iter_ptr);
-        for (int bin = lane; bin < ncand; bin += 32) {
-            float sc;
-            if (a.score_fn == CB_SCORE_COSINE) sc = (den[bin] > 1e-15f) ? num[bin] * rsqrtf(den[bin] + 1e-10f) : -3.0e38f;
-            else sc = num[bin];
+        for (int k = k0; k < V; k += parts) {
+            const int bin = lane * V + k;
+            if (bin >= ncand) continue;
+            float num = 0.0f, den = 0.0f;
+            for (int w = 0; w < parts; ++w) {
+                num += sc[(size_t)w * CB_SCORE_WARP_FLOATS + k * 32 + lane];
+                den += sc[(size_t)w * CB_SCORE_WARP_FLOATS + 256 + k * 32 + lane];
+            }
+            float s;
+            if (a.score_fn == CB_SCORE_COSINE) s = (den > 1e-15f) ? num * rsqrtf(den + 1e-10f) : -3.0e38f;
+            else s = num;
             const unsigned int gb = (unsigned int)(a.d.feat_off[f] + bin);
             if (noise_std > 0.0f) {
                 const unsigned long long h = cb_mix64(a.seed ^ cb_mix64((it << 8) + a.level) ^ ((unsigned long long)gb * 0x9E3779B97F4A7C15ull));
-                sc += cb_normal(h) * noise_std;
+                s += cb_normal(h) * noise_std;
             }
-            sc *= fw;
-            if (sc == sc) {
-                const unsigned long long key = ((unsigned long long)cb_float_to_ordered(sc) << 32) | (unsigned long long)(0xFFFFFFFFu - gb);
+            s *= fw;
+            if (s == s) {
+                const unsigned long long key = ((unsigned long long)cb_float_to_ordered(s) << 32) | (unsigned long long)(0xFFFFFFFFu - gb);
                 best = key > best ? key : best;
             }
         }
@@ -1202,8 +1218,7 @@ static __device__ void cb_score_finalize(const CbScoreArgs& a, int f, const floa
 
 // `red` is scratch shared memory of `red_floats` floats (the histogram tile is no longer needed at this point), at
 // least CB_SCORE_WARP_FLOATS per scoring warp.  With fewer features than warps several warps score one feature: they
-// split the leaves and the first of them adds the partial terms up, so the per-feature chain of dependent loads is
-// L / warps long instead of L.
+// split the parents, so the chain of dependent loads is parents / warps long, and then the rows of bins.
 // noise_in >= 0: the standard deviation of the score noise, already computed by the caller (it only depends on the
 // iteration, so the fused kernel computes it while the histogram phase runs); < 0: compute it here.
 static __device__ void cb_score_phase(const CbScoreArgs& a, int cta, int ncta, float* red, int red_floats,
@@ -1217,12 +1232,15 @@ static __device__ void cb_score_phase(const CbScoreArgs& a, int cta, int ncta, f
     }
     if (ts) ts[0] = cb_globaltimer();
     const int nf = a.f_end - a.f_begin;
-    const int L = 1 << a.level;
+    const int parents = a.level > 0 ? 1 << (a.level - 1) : 1;
     if (wpc < 1 || nf <= 0) return;
-    // warps per feature: as many as there are idle warps in the grid (power of two, at most one per leaf)
-    int wpf = 1;
-    while (wpf * 2 <= min(wpc, L) && (long long)nf * wpf * 2 <= (long long)ncta * wpc) wpf *= 2;
-    const int fpc = wpc / wpf;                           // features per block and round
+    // warps per feature: the count with the fewest pairs in a row for a warp, over all rounds (a round costs about one more)
+    int wpf = 1, fpc = wpc, best = 0x7fffffff;
+    for (int w = 1; w <= min(wpc, parents); w += (w + 1) >> 1) {
+        const int fit = wpc / w, rounds = (nf + ncta * fit - 1) / (ncta * fit);
+        const int cost = rounds * ((parents + w - 1) / w + 1);
+        if (cost < best) { best = cost; wpf = w; fpc = min(fit, (nf + ncta * rounds - 1) / (ncta * rounds)); }
+    }
     const int slot = warp / wpf, sub = warp - slot * wpf;
     float* sc = red + (size_t)warp * CB_SCORE_WARP_FLOATS;
     for (int fbase = a.f_begin + cta * fpc; fbase < a.f_end; fbase += ncta * fpc) {
@@ -1231,15 +1249,8 @@ static __device__ void cb_score_phase(const CbScoreArgs& a, int cta, int ncta, f
         if (have) cb_score_accumulate(a, f, sub, wpf, sc);
         if (ts) ts[1] = cb_globaltimer();
         if (wpf > 1) __syncthreads();
-        if (have && sub == 0) {
-            const int nb = a.d.feat_nb[f];
-            for (int w = 1; w < wpf; ++w) {
-                const float* o = sc + (size_t)w * CB_SCORE_WARP_FLOATS;
-                for (int bin = lane; bin < nb; bin += 32) { sc[bin] += o[bin]; sc[256 + bin] += o[256 + bin]; }
-            }
-            __syncwarp();
-            cb_score_finalize(a, f, sc, sc + 256, noise_std);
-        }
+        __syncwarp();
+        if (have) cb_score_finalize(a, f, red + (size_t)slot * wpf * CB_SCORE_WARP_FLOATS, wpf, sub, noise_std);
         if (wpf > 1) __syncthreads();
     }
     if (ts) ts[2] = cb_globaltimer();
