@@ -23,7 +23,6 @@ class LoopResult:
     best_iteration: Optional[int]
     best_score: Dict[str, Dict[str, float]]
     launches_per_iter: int = 0
-    train_approx: Optional[np.ndarray] = None
 
 
 class ObjectiveContext:
@@ -336,8 +335,7 @@ def run_boosting(o, objective, store, eval_stores, y_train, w_train, base_train,
                         else "Stopped by callback")
             break
     snap.finalize(dict(trees=trees, hist=hist.data, iters=hist.iters))
-    return LoopResult(trees, hist.data, best_it, _best_scores(hist, metrics), 0,
-                      approx[:, :n].t().double().cpu().numpy())
+    return LoopResult(trees, hist.data, best_it, _best_scores(hist, metrics), 0)
 
 
 class OrderedState:
@@ -864,7 +862,5 @@ def _run_fast(o, objective, store, eval_stores, y_train, w_train, base_train, ev
               "".join(f.kind[0] for f in store.features), file=sys.stderr)
         print("phase us per level [leaf update, histogram, grid wait, reduce + push, score, select]:\n",
               np.round(eng.phase_times_us(), 1), file=sys.stderr)
-    train_approx = (eng.approx[:, :n].t().double().cpu().numpy() if K > 1
-                    else eng.approx[:n].double().cpu().numpy().reshape(-1, 1))
     eng.close()
-    return LoopResult(trees, hist.data, best_it, _best_scores(hist, metrics), launches, train_approx)
+    return LoopResult(trees, hist.data, best_it, _best_scores(hist, metrics), launches)
