@@ -544,10 +544,12 @@ static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass
     // thread block (and at most 4096, which keeps two strides inside 32 bits)
     const long long nblk = (n + 2 * CB_LANE_THREADS - 1) / (2 * CB_LANE_THREADS);
     const int most = (int)(nblk < 1 ? 1 : (nblk < 4096 ? nblk : 4096));
-    // The leaves of two slot passes hold different numbers of documents, so passes as items of their own leave blocks waiting
-    // (10.5M x 28, two passes in one round of items: blocks finished between 98 and 230 us).  An item takes its chunk
-    // through all passes where there are chunks enough for every SM; a small shard spreads its passes over the SMs instead.
-    const int seq = nblk >= grid && nslots <= 256 ? 1 : 0;         // (a list entry has eight bits for the slot)
+    // A shard of many rows takes each chunk through all slot passes as one item: one scan, the other passes read its list, and
+    // blocks finish together although the leaves of two passes hold different numbers of documents.  A tile of 200 KB that
+    // every block zeroes, writes and has added up costs about 16 us, though, and the scan 0.7 ns a document and SM: below
+    // some 23K documents per SM the passes are items of their own, so that a block has one tile (400K x 39, 129 bins, level 7:
+    // 2.6 times the time with all passes in an item).
+    const int seq = nblk >= 14ll * grid && nslots <= 256 ? 1 : 0;         // (a list entry has eight bits for the slot)
     double W = 0.0;
     int min_items = 0;
     bool mixed = false;
@@ -559,7 +561,8 @@ static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass
         min_items += per[i];
         if (cost[i] != cost[0]) mixed = true;
     }
-    const int rounds = (mixed && p->a.h.work) ? 2 : 1;      // items of different times are handed out by a counter
+    // items of different times are handed out by a counter in two rounds, where a second tile per block is small change
+    const int rounds = (mixed && p->a.h.work && nblk >= 14ll * grid) ? 2 : 1;
     long long T = (long long)grid * rounds;
     while (T < min_items) T += grid;
     long long used = 0;
@@ -644,8 +647,10 @@ CB_API int cb_fused_geometry(CbFusedPlan* p, int level, int* slots_per_pass, int
     const long long n = p->a.h.d.n;
     if (level < CB_MAX_LEVELS) {
         p->lane_level[level] = 0;
+        // One feature group leaves three quarters of a 32-byte sector unread (10.5M x 4: 0.90 against 0.78 ms an iteration on
+        // the other path; 10.5M x 8: 0.90 against 0.85, 1.2M x 8 even, 100K x 8 0.28 against 0.30, from 12 columns on faster).
         // document and row numbers of that path are 32 bits wide, two work strides beyond the last document included
-        if (p->lanes && narrow && n < (1ll << 28)) {
+        if (p->lanes && narrow && n < (1ll << 28) && (G > 2 || (G == 2 && n < (1ll << 22)))) {
             const int grid = cb_fused_lane_geometry(p, level, slots_per_pass, smem_bytes, threads, chunks, copies, bundle);
             if (grid != 0) return grid > 0 ? grid : 0;
         }
