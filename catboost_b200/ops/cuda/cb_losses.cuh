@@ -40,14 +40,14 @@ __device__ __forceinline__ CbLossOut cb_loss_eval(int loss, float p0, float p1, 
         }
         case CB_LOSS_LOGLOSS:
         case CB_LOSS_CROSSENTROPY: {
-            float p = 1.0f / (1.0f + __expf(-a));
-            o.der = y - p;
-            o.hess = fmaxf(p * (1.0f - p), 1e-16f);
-            // log(1+e^a) - y a, stable for both signs
-            // softplus, stable for both signs; the fast logarithm is off by at most 6e-8 per document (the reported loss
-            // is a mean of these)
-            float sp = fmaxf(a, 0.0f) + __logf(1.0f + __expf(-fabsf(a)));
-            o.value = sp - y * a;
+            // one exponential and one reciprocal serve the probability, its product with 1 - p (without the cancellation)
+            // and the softplus, stable for both signs; the fast logarithm is off by at most 6e-8 per document (the
+            // reported loss is a mean of these)
+            const float e = __expf(-fabsf(a));
+            const float r = __fdividef(1.0f, 1.0f + e), er = e * r;
+            o.der = y - (a >= 0.0f ? r : er);
+            o.hess = fmaxf(er * r, 1e-16f);
+            o.value = fmaxf(a, 0.0f) + __logf(1.0f + e) - y * a;
             break;
         }
         case CB_LOSS_POISSON: {

@@ -30,8 +30,8 @@ def _engine(store, y, depth, lane_hist, **kw):
 
 
 @pytest.mark.parametrize("n,widths,depth,sparse", [
-    (1, [5], 1, False),
-    (255, [2, 3, 200], 3, False),
+    (1, [5] * 5, 1, False),
+    (255, [2, 3, 200, 7, 9], 3, False),
     (1023, [17] * 8, 4, False),                      # one row block of two groups: 16 documents a load
     (1025, [129] * 9, 6, False),                     # three groups: 8 documents a load
     (30_011, [129] * 28, 6, False),                  # seven groups: 4 documents a load, several slot passes
@@ -101,3 +101,36 @@ def test_lane_pass_grows_the_trees_of_the_other_pass(n, F, borders, depth):
     same = (outs[0][0][0, :, :2] == outs[1][0][0, :, :2]).all(-1)
     assert same[: min(depth, 5)].all(), (outs[0][0][0], outs[1][0][0])
     assert np.allclose(outs[0][3], outs[1][3], rtol=5e-3)
+
+
+@pytest.mark.parametrize("n,weighted,steps", [(1, False, 1), (33, True, 3), (40_001, False, 3), (40_001, True, 1)])
+def test_logloss_leaf_steps_equal_newton_steps_in_64_bits(n, weighted, steps):
+    """Logloss leaves: every step, the first included, adds fixed-point values scaled by the loss's own bounds."""
+    from catboost_b200.train.objectives import make_objective
+    from catboost_b200.train.gpu_engine import GpuObliviousEngine
+    store, cols = _store(n, [33] * 6, seed=n)
+    rng = np.random.default_rng(n)
+    y = (rng.random(n) < 1.0 / (1.0 + np.exp(-(cols[0] / 8.0 - 2.0)))).astype(np.float32)
+    w = (rng.random(n) * 1000.0).astype(np.float32) if weighted else np.ones(n, dtype=np.float32)
+    start = (3.0 * rng.standard_normal(n)).astype(np.float32)
+    eng = GpuObliviousEngine(store, torch.from_numpy(y), torch.from_numpy(w) if weighted else None, torch.from_numpy(start),
+                             make_objective("Logloss", {}), depth=4, iterations=2, learning_rate=1.0, l2_leaf_reg=3.0,
+                             random_strength=0.0, bootstrap_type="No", leaf_iterations=steps, leaf_backtracking="No", lane_hist=True)
+    eng.step(1)
+    torch.cuda.synchronize()
+    leaf = eng.leaf[:n].cpu().numpy().astype(np.int64) & 0xFFFF
+    delta = np.zeros(16)
+    for _ in range(steps):
+        p = 1.0 / (1.0 + np.exp(-(start.astype(np.float64) + delta[leaf])))
+        der, hess = np.zeros(16), np.zeros(16)
+        np.add.at(der, leaf, w * (y - p))
+        np.add.at(hess, leaf, w * p * (1.0 - p))
+        delta += der / (hess + 3.0)
+    weights = np.zeros(16)
+    np.add.at(weights, leaf, w.astype(np.float64))
+    # a probability is right to a few 1e-7 (fast exponential), a sum of up to n of them to no more of its mass; the steps divide
+    # two such sums
+    assert np.allclose(eng.model_vals[0].cpu().numpy(), delta, rtol=5e-6, atol=5e-6 * max(1.0, np.abs(delta).max()))
+    assert np.allclose(eng.model_wts[0].cpu().numpy(), weights, rtol=1e-6)
+    eng.finish()
+    eng.close()
