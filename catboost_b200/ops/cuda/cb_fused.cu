@@ -2,7 +2,8 @@
 //   (0) the leaf-index update for the split chosen at the previous level (inside the histogram pass when the
 //       bundled path runs: the pass has the bin words of its documents in registers anyway),
 //   (A) streaming histogram accumulation of the local rows (shared-memory integer atomics, one slot per parent
-//       leaf: only the lighter child is accumulated, the sibling is parent - child),
+//       leaf: only the lighter child is accumulated, the sibling is parent - child); two-statistic fixed-point levels
+//       of three or more feature groups keep every feature in a bank of its own (cb_lanes.cuh),
 //   (B) the reduce-scatter: every rank sums its chunk tiles and stores the feature slice that rank r owns straight
 //       into rank r's slot buffer over NVLink as tagged 8-byte words (value + level tag),
 //   (C) on the owner: the score phase polls the words it needs until they carry this level's tag (bounded), sums the
