@@ -144,15 +144,16 @@ class GpuPredictor:
         res = np.empty((n, self.dims), dtype=np.float64) if out is None else out
         if n == 0:
             return res
-        if chunk_rows <= 0:
-            # 16 MB of floats per buffer, so that filling a buffer, its copy and its kernel overlap from 1M values on (1M x
-            # 28 rows, 500 trees: 7.9 ms with one 256 MB buffer); one geometry for every batch above 64K rows, so that the
-            # buffers kept from the previous call fit the next one whatever its length
-            chunk_rows = max(4096, (4 << 20) // max(F, 1)) if n > 65536 else n
         xt = torch.from_numpy(X)
         src_pinned = bool(xt.is_pinned())            # the caller's rows are page-locked: no staging copy needed
+        if chunk_rows <= 0:
+            # 16 MB of floats per buffer, so that filling a buffer, its copy and its kernel overlap from 1M values on (1M x
+            # 28 rows, 500 trees: 7.9 ms with one 256 MB buffer); page-locked rows, where nothing is filled, go 256 MB at a
+            # time.  One geometry for every batch above 64K rows, so that the buffers kept from the previous call fit the
+            # next one whatever its length
+            chunk_rows = max(4096, ((64 if src_pinned else 4) << 20) // max(F, 1)) if n > 65536 else n
         with torch.cuda.device(self.dev):
-            nbuf = 3 if n > 65536 else (2 if n > chunk_rows else 1)
+            nbuf = (2 if src_pinned else 3) if n > 65536 else (2 if n > chunk_rows else 1)
             key = (chunk_rows, F, src_pinned, nbuf)
             bufs = self.__dict__.setdefault("_bufs", {}).get(key)
             if bufs is None:
