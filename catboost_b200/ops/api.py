@@ -200,8 +200,7 @@ def leaf_newton(loss_id: int, p0: float, p1: float, approx: torch.Tensor, target
     w = None if weight is None else weight.contiguous().float()
     bt = {"No": 0, "AnyImprovement": 1, "Armijo": 2}[str(backtracking or "No")]
     rc = lib.cb_leaf_newton(int(loss_id), float(p0), float(p1), _p(a), _p(t), _p(w), _p(leaf), int(n), L, _p(delta), _p(sums),
-                            _p(counter), _p(vmax), 1.0 if w is None else 0.0, int(steps), 1 if newton else 0, float(l2), float(lr),
-                            _p(cur), None, None, L,
+                            _p(counter), _p(vmax), int(steps), 1 if newton else 0, float(l2), float(lr), _p(cur), None, None, L,
                             _p(iter_ptr), _p(leaf_w), None, bt, grid, _stream(dev))
     if rc == -2:
         return None

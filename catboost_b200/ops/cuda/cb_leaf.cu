@@ -22,9 +22,10 @@
 // is not known yet) and records max |w der|, max |w hess|; later steps use fixed point with native integer atomics:
 // one int32 cell per (leaf, statistic, replica), scaled so that twice the recorded bound times the number of documents
 // a replica can receive stays below 2^31 (about 21 bits per value with 32 replicas at 10M documents -- finer than what
-// an fp32 running sum keeps).  A value beyond the bound goes to the double accumulator directly.  Logloss needs no recorded
-// bound (|der| <= weight, hess <= weight / 4), so its first step uses these cells as well (10.5M documents, 10 steps: the
-// launch took 374 us with an fp32 first step).
+// an fp32 running sum keeps).  A value beyond the bound goes to the double accumulator directly.  Logloss bounds its
+// derivatives by the document weight, but cells scaled by that bound lose what is far below it (10.5M documents: leaf
+// values off by 2e-2 at margins N(-15, 0.5) and by 3e-2 with lognormal(0, 3) weights, whose leaf weights are off by 2e-3),
+// so every loss takes its first step in fp32 and learns the scale there (22 to 33 us of a tree at 10.5M documents).
 #include "cb_common.cuh"
 #include "cb_losses.cuh"
 #include "cb_comm.cuh"
@@ -47,7 +48,6 @@ struct CbLeafNewtonArgs {
     float* cur_vals;         // [L] lr * delta after the last step
     float* model_vals; float* model_wts; int Lstride; const int* iter_ptr;
     float* leaf_w;           // [L] per-leaf weight sums
-    float wmax;              // largest document weight (0: not known)
     int backtrack;           // CbBacktrack
     CbComm c;
 };
@@ -90,7 +90,6 @@ __global__ void __launch_bounds__(512, 2) cb_leaf_newton_kernel(CbLeafNewtonArgs
     const long long n4 = (a.n + 3) >> 2;
     const long long stride = (long long)gridDim.x * blockDim.x;
     const bool can_quant = (a.n / gridDim.x) < (1ll << 22);
-    const bool bounded = LOSS == CB_LOSS_LOGLOSS && a.wmax > 0.0f;
     // documents one replica of a cell can receive: those of the threads that share the replica index
     const long long per_thread = ((n4 + stride - 1) / stride) * 4;
     const float qcap = fminf(8388607.0f, floorf(2147483647.0f / (float)(per_thread * (blockDim.x / C) + 1)) - 1.0f);
@@ -98,15 +97,9 @@ __global__ void __launch_bounds__(512, 2) cb_leaf_newton_kernel(CbLeafNewtonArgs
     float cur_step = 1.0f;
     for (int step = 0; step < a.steps; ++step) {
         const bool first = step == 0, last = step == a.steps - 1;
-        const bool quant = (!first || bounded) && can_quant;
-        float M0 = 0.f, M1 = 0.f, sc0 = 0.f, sc1 = 0.f, sc2 = 0.f;
-        if (bounded) {
-            M0 = 1.0001f * a.wmax;                   // (a hair more: at the start every document may sit on the bound)
-            M1 = 0.25f * M0;
-            sc0 = qcap / M0;
-            sc1 = qcap / M1;
-            sc2 = exp2f(floorf(__log2f(sc0)));       // a power of two: counts and round weights are exact
-        } else if (quant) {
+        const bool quant = !first && can_quant;
+        float M0 = 0.f, M1 = 0.f, sc0 = 0.f, sc1 = 0.f;
+        if (quant) {
             M0 = 2.0f * fmaxf(__ldcg(a.vmax), 1e-30f);
             M1 = 2.0f * fmaxf(__ldcg(a.vmax + 1), 1e-30f);
             sc0 = qcap / M0;
@@ -144,11 +137,9 @@ __global__ void __launch_bounds__(512, 2) cb_leaf_newton_kernel(CbLeafNewtonArgs
                         int* cell = si + (size_t)(l * 4) * C + lane_copy;
                         atomicAdd(cell, __float2int_rn(vd * sc0));
                         atomicAdd(cell + C, __float2int_rn(vh * sc1));
-                        if (first) atomicAdd(cell + 2 * C, __float2int_rn(w * sc2));
                     } else {
                         atomicAdd(&S[3 * l], (double)vd);
                         atomicAdd(&S[3 * l + 1], (double)vh);
-                        if (first) atomicAdd(&S[3 * l + 2], (double)w);
                     }
                 } else {
                     float* cell = sl + (size_t)(l * 4) * C + lane_copy;
@@ -156,14 +147,13 @@ __global__ void __launch_bounds__(512, 2) cb_leaf_newton_kernel(CbLeafNewtonArgs
                     atomicAdd(cell + C, vh);
                     if (first) {
                         atomicAdd(cell + 2 * C, w);
-                        if (bounded) continue;
                         mx0 = fmaxf(mx0, fabsf(vd));
                         mx1 = fmaxf(mx1, fabsf(vh));
                     }
                 }
             }
         }
-        if (first && !bounded) {
+        if (first) {
             for (int off = 16; off > 0; off >>= 1) {
                 mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, off));
                 mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, off));
@@ -184,14 +174,13 @@ __global__ void __launch_bounds__(512, 2) cb_leaf_newton_kernel(CbLeafNewtonArgs
             if (t != 0.0) atomicAdd(&S[3 * L], t);
         }
         if (quant) {
-            const double inv0 = 1.0 / (double)sc0, inv1 = 1.0 / (double)sc1;
-            const int per = first ? 3 : 2;           // statistics of a leaf in this step
-            for (int i = threadIdx.x; i < per * L; i += blockDim.x) {
-                const int l = i / per, s2 = i - per * l;
+            const double inv0 = (double)M0 / (double)qcap, inv1 = (double)M1 / (double)qcap;
+            for (int i = threadIdx.x; i < 2 * L; i += blockDim.x) {
+                const int l = i >> 1, s2 = i & 1;
                 const int* ph = si + (size_t)(l * 4 + s2) * C;
                 long long qq = 0;
                 for (int c = 0; c < C; ++c) qq += ph[c];
-                if (qq != 0) atomicAdd(&S[3 * l + s2], (double)qq * (s2 == 0 ? inv0 : (s2 == 1 ? inv1 : 1.0 / (double)sc2)));
+                if (qq != 0) atomicAdd(&S[3 * l + s2], (double)qq * (s2 ? inv1 : inv0));
             }
         } else {
             for (int i = threadIdx.x; i < 3 * L; i += blockDim.x) {
@@ -356,12 +345,12 @@ CB_API int cb_leaf_newton_max_grid(int L) {
 
 CB_API int cb_leaf_newton(int loss, float p0, float p1, const float* approx, const float* target, const float* weight,
                           const unsigned short* leaf, long long n, int L, float* delta, double* sums,
-                          unsigned int* counter, float* vmax, float wmax,
+                          unsigned int* counter, float* vmax,
                           int steps, int newton, float l2, float lr, float* cur_vals, float* model_vals,
                           float* model_wts, int Lstride, const int* iter_ptr, float* leaf_w, const CbComm* comm,
                           int backtrack, int grid, cudaStream_t st) {
     CbLeafNewtonArgs a{loss, p0, p1, approx, target, weight, leaf, n, L, delta, sums, counter, vmax, steps, newton, l2, lr,
-                       cur_vals, model_vals, model_wts, Lstride, iter_ptr, leaf_w, wmax, backtrack, CbComm()};
+                       cur_vals, model_vals, model_wts, Lstride, iter_ptr, leaf_w, backtrack, CbComm()};
     if (comm) a.c = *comm; else { a.c.nranks = 1; a.c.rank = 0; }
     int smem = 0;
     const int C = cb_leaf_newton_cells(L, &smem);

@@ -181,8 +181,8 @@ _SIGS = {
                             c_void_p, c_int, c_void_p]),
     "cb_leaf_newton_max_grid": (c_int, [c_int]),
     "cb_leaf_newton": (c_int, [c_int, c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_void_p,
-                               c_void_p, c_void_p, c_void_p, c_float, c_int, c_int, c_float, c_float, c_void_p, c_void_p,
-                               c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
+                               c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_void_p, c_int,
+                               c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "cb_leaf_newton_sums_doubles": (c_int, [c_int]),
     "cb_leaf_newton_msg_bytes": (c_int, [c_int]),
     "cb_iter_end": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p]),

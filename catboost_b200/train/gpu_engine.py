@@ -456,7 +456,7 @@ class GpuObliviousEngine:
             # all steps of the leaf estimation in one cooperative launch
             rc = lib.cb_leaf_newton(self.loss_id, self.p0, self.p1, _p(self.approx), _p(self.target), _p(self.weight),
                                    _p(self.leaf), self.n, self.L, _p(self.delta), _p(self.sums), _p(self.counter),
-                                   _p(self.leaf_vmax), self.weight_max,
+                                   _p(self.leaf_vmax),
                                    self.leaf_iterations, self.leaf_newton, self.l2, self.lr, _p(self.cur_vals),
                                    _p(self.model_vals), _p(self.model_wts), self.L, _p(self.iter_ptr), _p(self.leaf_w),
                                    comm, self.leaf_backtracking, self.leaf_grid, self._stream())

@@ -134,3 +134,38 @@ def test_logloss_leaf_steps_equal_newton_steps_in_64_bits(n, weighted, steps):
     assert np.allclose(eng.model_wts[0].cpu().numpy(), weights, rtol=1e-6)
     eng.finish()
     eng.close()
+
+
+@pytest.mark.parametrize("shift,spread,weights,steps", [
+    (-13.0, 1.0, "", 1), (-13.0, 1.0, "", 3), (-15.0, 0.5, "", 3),       # documents that the model is sure of
+    (0.0, 3.0, "lognormal", 1), (0.0, 3.0, "one heavy", 1),              # documents far lighter than the heaviest one
+])
+def test_logloss_leaf_steps_keep_small_derivatives_and_weights(shift, spread, weights, steps):
+    """Leaf values and leaf weights of documents whose derivative or weight is orders below the largest possible one."""
+    from catboost_b200.train.objectives import make_objective
+    from catboost_b200.train.gpu_engine import GpuObliviousEngine
+    n = 40_001
+    store, _ = _store(n, [33] * 6, seed=5)
+    rng = np.random.default_rng(6)
+    y = np.zeros(n, dtype=np.float32) if shift < 0 else (rng.random(n) < 0.4).astype(np.float32)
+    w = {"": np.ones(n), "lognormal": np.exp(3.0 * rng.standard_normal(n)),
+         "one heavy": np.where(np.arange(n) == 7, 1.0e7, 1.0)}[weights].astype(np.float32)
+    start = (shift + spread * rng.standard_normal(n)).astype(np.float32)
+    eng = GpuObliviousEngine(store, torch.from_numpy(y), torch.from_numpy(w) if weights else None, torch.from_numpy(start),
+                             make_objective("Logloss", {}), depth=4, iterations=2, learning_rate=1.0, l2_leaf_reg=3.0,
+                             random_strength=0.0, bootstrap_type="No", leaf_iterations=steps, leaf_backtracking="No", lane_hist=True)
+    eng.step(1)
+    torch.cuda.synchronize()
+    leaf = eng.leaf[:n].cpu().numpy().astype(np.int64) & 0xFFFF
+    delta = np.zeros(16)
+    for _ in range(steps):
+        p = 1.0 / (1.0 + np.exp(-(start.astype(np.float64) + delta[leaf])))
+        der = np.bincount(leaf, w * (y - p), 16)
+        delta += der / (np.bincount(leaf, w * p * (1.0 - p), 16) + 3.0)
+    # a fast exponential of a margin of 15 is right to 1e-6, the sums add fewer than 2^12 such values each
+    got, wts = eng.model_vals[0].cpu().numpy(), eng.model_wts[0].cpu().numpy()
+    light = np.bincount(leaf, w.astype(np.float64), 16)
+    assert np.linalg.norm(got - delta) <= 5e-6 * np.linalg.norm(delta), np.abs(got / delta - 1.0).max()
+    assert np.allclose(wts, light, rtol=1e-6), np.abs(wts / light - 1.0).max()
+    eng.finish()
+    eng.close()
