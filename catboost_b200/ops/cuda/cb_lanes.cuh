@@ -414,8 +414,9 @@ cb_lane_cap_kernel(CbData d, const uint32_t* lanes, const short* ldom, const CbB
         __syncthreads();
         int best = 0;
         if (lane < bd.gcnt * 4) {
+            // (a padding column, dom < 0, holds every document in bin 0; nobody reads its cells, so they may wrap around)
             const int dom = ldom[bd.g0 * 4 + lane];
-            for (int bin = warp; bin < bd.B; bin += CB_LANE_THREADS / 32)
+            for (int bin = warp; bin < bd.B && dom >= 0; bin += CB_LANE_THREADS / 32)
                 if (bin != dom) best = max(best, cb_lane_sh[bin * 32 + lane]);
         }
         best = __reduce_max_sync(0xffffffffu, best);

@@ -169,3 +169,46 @@ def test_logloss_leaf_steps_keep_small_derivatives_and_weights(shift, spread, we
     assert np.allclose(wts, light, rtol=1e-6), np.abs(wts / light - 1.0).max()
     eng.finish()
     eng.close()
+
+
+def _sure_engine(store, n, depth=1, p=1.0e-4, positives=0.01, **kw):
+    """Logloss at a constant cursor: every negative's derivative is -p, the positives' is 1 - p."""
+    from catboost_b200.train.gpu_engine import GpuObliviousEngine
+    from catboost_b200.train.objectives import make_objective
+    y = (torch.rand(n, generator=torch.Generator(device="cuda").manual_seed(1), device="cuda") < positives).float()
+    args = dict(depth=depth, iterations=2, learning_rate=0.5, l2_leaf_reg=3.0, random_strength=0.0, bootstrap_type="No",
+                leaf_iterations=1, seed=3, lane_hist=True)
+    args.update(kw)
+    return GpuObliviousEngine(store, y, None, torch.full((n,), float(np.log(p / (1.0 - p)))), make_objective("Logloss", {}), **args), y
+
+
+def _negative_mass_error(eng, store, y, n, features):
+    """Level 0: largest error of a bin's derivative sum, over the mass of the bin's negatives."""
+    der = eng.stats[0, :n].double()
+    off, worst = store.feat_off_host, 0.0
+    for f in features:
+        nb = int(store.feat_nb_host[f])
+        bins = store.column(f)[:n].long()
+        exact = torch.bincount(bins, der, nb)
+        mass = torch.bincount(bins, der.abs() * (y < 0.5), nb)
+        got = eng.slots[off[f]: off[f] + nb].double()
+        full = mass > 0
+        worst = max(worst, float(((got - exact).abs()[full] / mass[full]).max()))
+    return worst
+
+
+@pytest.mark.parametrize("F", [5, 9, 30, 32])
+def test_padding_columns_leave_the_scale_alone(F):
+    """A last feature group of fewer than four columns: its padding columns hold every document in one bin."""
+    n = 2_000_003
+    store, _ = _store(n, [129] * F, seed=F)
+    eng, y = _sure_engine(store, n)
+    eng.step(1)
+    torch.cuda.synchronize()
+    steps = (n + 1663) // 1664
+    cap = -(-steps // eng.level_geo[0][4]) * 52 + 1            # documents of a lane total: more than any of 129 bins gets
+    quantum = 1.0 / (2.0 ** 31 / (cap + 1) - 1.0)
+    # half a quantum a negative, and fp32 sums of positives that weigh 100 times as much
+    assert _negative_mass_error(eng, store, y, n, (0, F - 1)) <= 0.5 * quantum / 1.0e-4 + 100 * 2.0 ** -20
+    eng.finish()
+    eng.close()
