@@ -310,6 +310,7 @@ __global__ void __launch_bounds__(LANES ? CB_LANE_THREADS : 1024, 1) cb_level_fu
 
 // ---- host side ---------------------------------------------------------------------------------------
 #define CB_MAX_LEVELS 16
+#define CB_LANE_SEQ_DOCS 23296                 // (14 steps of a thread block)
 struct CbFusedPlan {
     CbFusedArgs a;
     int threads;
@@ -331,6 +332,8 @@ struct CbFusedPlan {
     const uint32_t* lanes;
     const short* ldom;
     cudaStream_t lane_stream;                  // the stream the lane store was made on; the work lists go there too
+    std::vector<float> group_share;            // see cb_lane_plan (empty: a bin may hold every document)
+    long long seq_docs;                        // documents per SM from which a work item takes its chunk through all slot passes
     int lane_smem;                             // dynamic shared memory one block of that kernel may use
     int lane_level[CB_MAX_LEVELS];             // 1: the level takes that path
     long long lane_priv[CB_MAX_LEVELS];        // floats of its private tiles
@@ -386,7 +389,7 @@ CB_API CbFusedPlan* cb_fused_create(const CbData* d, const CbComm* comm, unsigne
     cudaDeviceGetAttribute(&p->sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
     p->sm_smem -= 2 * (int)fa.sharedSizeBytes;
     p->max_bundle = 0;
-    p->lanes = nullptr; p->ldom = nullptr; p->lane_stream = nullptr;
+    p->lanes = nullptr; p->ldom = nullptr; p->lane_stream = nullptr; p->seq_docs = CB_LANE_SEQ_DOCS;
     cudaFuncAttributes fl;
     if (cudaFuncGetAttributes(&fl, cb_level_fused_kernel<true>) != cudaSuccess) { cudaGetLastError(); delete p; return nullptr; }
     p->lane_smem = p->max_smem + (int)fa.sharedSizeBytes - (int)fl.sharedSizeBytes;
@@ -460,6 +463,8 @@ CB_API void cb_fused_set_lanes(CbFusedPlan* p, const uint32_t* lanes, const shor
     p->ldom = ldom;
     p->lane_stream = st;
 }
+// share[g]: see cb_lane_plan, host memory
+CB_API void cb_fused_set_lane_share(CbFusedPlan* p, const float* share, int G) { p->group_share.assign(share, share + G); }
 // Floats of private tiles the level needs when it takes the feature-per-lane path (0: it does not).
 CB_API long long cb_fused_lane_priv(CbFusedPlan* p, int level) {
     return level < CB_MAX_LEVELS && p->lane_level[level] ? p->lane_priv[level] : 0;
@@ -474,19 +479,42 @@ CB_API void cb_fused_set_lane_list(CbFusedPlan* p, int2* q, unsigned int* row) {
     p->a.h.list_row = row;
 }
 
-// Feature-per-lane geometry of one level: grid size, 0 = take the other path, -1 = error.
-static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass, int* smem_bytes, int* threads, int* chunks,
-                                  int* copies, int* bundle) {
+// ---- feature-per-lane path: what a level does, worked out on the host from sizes alone -------------------------------
+struct CbLanePlan {
+    std::vector<CbBundle> bundles;
+    std::vector<double> cost;          // of a bundle
+    std::vector<int2> items;
+    std::vector<unsigned int> cap;     // documents a lane total can receive
+    std::vector<unsigned int> limit;   // documents a cell may receive
+    int smem = 0, chunks = 0;
+    long long priv = 0, list = 0;      // floats of private tiles, document list entries
+};
+
+// Documents one cell may receive.  The fixed-point scale is 2^31 / (documents of the fullest cell), so this is the number of
+// steps a statistic's range is cut into: values much smaller than the largest one all round the same way when the steps are
+// coarse (0.5 % positives: the derivative of a negative is 20 steps at 2^19 documents a cell, 320 at 2^15).  2^17 leaves
+// 16383 steps and 2^15 65534; the per-group path's chunks of 2^19 documents leave 4094 per replica of a cell, and it has one
+// where there are many leaves, two where there are few.  What a chunk costs is its tiles (200 KB: about 16 us to zero, write
+// and add up, as much as streaming 16K documents), so the limit follows their size: between 2^15 and 2^17.
+static unsigned int cb_lane_cell_limit(long long tile_bytes) {
+    const double v = 65536.0 * (double)tile_bytes / 200000.0;
+    return v < 32768.0 ? 32768u : (v > 131072.0 ? 131072u : (unsigned int)v);
+}
+
+// gb[g]: padded bins of the widest feature of group g; share[g]: largest share of the documents that one bin of the group
+// holds, the most frequent bin of every feature left out.  False: the level takes the other path.
+static bool cb_lane_plan(CbLanePlan& out, long long n, int G, const int* gb, const float* share, int level, int grid, int lane_smem,
+                         bool counter, long long seq_docs) {
     const int nslots = level == 0 ? 1 : (1 << (level - 1));
-    const int G = p->a.h.d.G;
-    const long long n = p->a.h.d.n;
-    auto gb = [&](int g) { return p->group_bins.empty() ? p->a.h.B : p->group_bins[g]; };
-    const int ints = p->lane_smem / 4 - cb_lane_extra_ints(0);
+    const int ints = lane_smem / 4 - cb_lane_extra_ints(0);
+    std::vector<CbBundle>& bundles = out.bundles;
+    std::vector<double>& cost = out.cost;
+    bundles.clear(); cost.clear(); out.items.clear(); out.cap.clear(); out.limit.clear();
     // Cost of streaming 32 documents through a bundle: a fixed part per slot pass and a part per document taken.
     const double taken = level == 0 ? 32.0 : 15.0;
     auto shape = [&](int g, int gc, CbBundle* b) {
         int B = 4;
-        for (int q = 0; q < gc; ++q) B = gb(g + q) > B ? gb(g + q) : B;
+        for (int q = 0; q < gc; ++q) B = gb[g + q] > B ? gb[g + q] : B;
         const int FL = gc > 4 ? 32 : (gc > 2 ? 16 : 8);
         const int per = B * (FL == 32 ? 64 : 32) + 64;
         int spp = ints / per;
@@ -498,8 +526,6 @@ static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass
         *b = CbBundle{g, gc, B, 1, spp, np, 1, FL, 0, 0, 0, 0, 0};
         return np * 25.0 + taken * (FL == 32 ? 3.2 : (FL == 16 ? 2.2 : 1.2));
     };
-    std::vector<CbBundle> bundles;
-    std::vector<double> cost;
     for (int g = 0; g < G; g += 8) {
         const int gc = G - g < 8 ? G - g : 8;
         // a row block is one bundle, or is cut into halves (quarters) where a narrower tile saves enough slot passes
@@ -526,10 +552,11 @@ static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass
         if (cw <= sum) { bundles.push_back(w); cost.push_back(cw); }
         else for (size_t i = 0; i < cut.size(); ++i) { bundles.push_back(cut[i]); cost.push_back(ccut[i]); }
     }
-    for (double c : cost) if (c >= 1e29) return 0;
+    for (double c : cost) if (c >= 1e29) return false;
     const int nbun = (int)bundles.size();
-    if (nbun < 1 || nbun > 0xFFFF) return 0;
-    int smem = 0;
+    if (nbun < 1 || nbun > 0xFFFF) return false;
+    int& smem = out.smem;
+    smem = 0;
     for (const CbBundle& b : bundles) {
         const int need = (b.spp * b.B * (b.FL == 32 ? 64 : 32) + cb_lane_extra_ints(b.spp)) * 4;
         if (need > smem) smem = need;
@@ -537,10 +564,6 @@ static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass
     // the score phase reuses the tile as scratch; one block per SM runs either way, so every warp gets some
     const int want = (CB_LANE_THREADS / 32) * CB_SCORE_WARP_FLOATS * 4;
     if (smem < want) smem = want;
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cb_level_fused_kernel<true>, CB_LANE_THREADS, smem) != cudaSuccess) { cudaGetLastError(); return -1; }
-    if (occ < 1) return 0;
-    const int grid = p->sm_count;                      // one block per SM
     // chunks: every item about the same time, their number a whole multiple of the grid; no more chunks than steps of a
     // thread block (and at most 4096, which keeps two strides inside 32 bits)
     const long long nblk = (n + 2 * CB_LANE_THREADS - 1) / (2 * CB_LANE_THREADS);
@@ -550,27 +573,35 @@ static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass
     // every block zeroes, writes and has added up costs about 16 us, though, and the scan 0.7 ns a document and SM: below
     // some 23K documents per SM the passes are items of their own, so that a block has one tile (400K x 39, 129 bins, level 7:
     // 2.6 times the time with all passes in an item).
-    const int seq = nblk >= 14ll * grid && nslots <= 256 ? 1 : 0;         // (a list entry has eight bits for the slot)
+    const bool many = n >= seq_docs * grid;
+    const int seq = many && nslots <= 256 ? 1 : 0;     // (a list entry has eight bits for the slot)
     double W = 0.0;
-    int min_items = 0;
+    long long min_items = 0;
     bool mixed = false;
-    std::vector<int> per(nbun);                        // items a chunk of the bundle takes
+    std::vector<int> per(nbun), least(nbun);           // items a chunk of the bundle takes; fewest chunks
     for (int i = 0; i < nbun; ++i) {
         bundles[i].seq = seq;
         per[i] = seq ? 1 : bundles[i].npass;
         W += cost[i];
-        min_items += per[i];
+        // chunks small enough that no cell receives more documents than it may (a lane total has a 32nd of them all)
+        float sh = 1.0f / 32.0f;
+        for (int q = 0; q < bundles[i].gcnt; ++q) sh = share[bundles[i].g0 + q] > sh ? share[bundles[i].g0 + q] : sh;
+        out.limit.push_back(cb_lane_cell_limit((long long)nslots * bundles[i].B * (bundles[i].FL == 32 ? 64 : 32) * 4));
+        const double k = (double)n * sh / (double)out.limit[i];
+        least[i] = k < 1.0 ? 1 : (k > (double)most ? most : (int)k + 1);
+        if (least[i] > most) least[i] = most;
+        min_items += (long long)least[i] * per[i];
         if (cost[i] != cost[0]) mixed = true;
     }
     // items of different times are handed out by a counter in two rounds, where a second tile per block is small change
-    const int rounds = (mixed && p->a.h.work && nblk >= 14ll * grid) ? 2 : 1;
+    const int rounds = (mixed && counter && many) ? 2 : 1;
     long long T = (long long)grid * rounds;
     while (T < min_items) T += grid;
     long long used = 0;
     for (int i = 0; i < nbun; ++i) {
         const double each = cost[i] / per[i];
         int k = (int)((double)T * each / W);
-        k = k < 1 ? 1 : (k > most ? most : k);
+        k = k < least[i] ? least[i] : (k > most ? most : k);
         bundles[i].nK = k;
         used += (long long)k * per[i];
     }
@@ -586,9 +617,11 @@ static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass
         ++bundles[pick].nK;
         used += per[pick];
     }
-    int best = 1, unit = 0;
-    long long priv = 0, list = 0;
-    std::vector<unsigned int> cap(nbun);
+    int unit = 0;
+    int& best = out.chunks;
+    long long &priv = out.priv, &list = out.list;
+    best = 1; priv = list = 0;
+    out.cap.resize(nbun);
     for (int i = 0; i < nbun; ++i) {
         CbBundle& b = bundles[i];
         if (b.nK > best) best = b.nK;
@@ -601,9 +634,9 @@ static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass
         b.list0 = list;
         if (b.seq && b.npass > 1) list += (long long)b.nK * b.list_stride;
         // documents one lane total can receive
-        cap[i] = (unsigned int)(((nblk + b.nK - 1) / b.nK) * (2 * CB_LANE_THREADS / 32) + 1);
+        out.cap[i] = (unsigned int)(((nblk + b.nK - 1) / b.nK) * (2 * CB_LANE_THREADS / 32) + 1);
     }
-    std::vector<int2> items;
+    std::vector<int2>& items = out.items;
     std::vector<int> order(nbun);
     for (int i = 0; i < nbun; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
@@ -613,30 +646,79 @@ static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass
         for (int bi : order)
             if (k < bundles[bi].nK)
                 for (int ps = 0; ps < per[bi]; ++ps) items.push_back(make_int2(bi | (ps << 16), k));
-    if (p->d_btab[level]) { cudaFree(p->d_btab[level]); p->d_btab[level] = nullptr; }
-    if (p->d_items[level]) { cudaFree(p->d_items[level]); p->d_items[level] = nullptr; }
-    if (p->d_cap[level]) { cudaFree(p->d_cap[level]); p->d_cap[level] = nullptr; }
-    if (cudaMalloc(&p->d_btab[level], bundles.size() * sizeof(CbBundle)) != cudaSuccess ||
-        cudaMalloc(&p->d_items[level], items.size() * sizeof(int2)) != cudaSuccess ||
-        cudaMalloc(&p->d_cap[level], (size_t)nbun * sizeof(unsigned int)) != cudaSuccess) { cudaGetLastError(); return -1; }
+    return true;
+}
+
+// The same from sizes alone: document chunks and feature groups of every bundle; returns their number (0: the level takes the
+// other path).
+CB_API int cb_lane_plan_query(long long n, int G, const int* group_bins, const float* share, int level, int grid, int lane_smem,
+                              int max_bundles, int* chunks, int* groups) {
+    CbLanePlan lp;
+    if (!cb_lane_plan(lp, n, G, group_bins, share, level, grid, lane_smem, true, CB_LANE_SEQ_DOCS)) return 0;
+    for (int i = 0; i < (int)lp.bundles.size() && i < max_bundles; ++i) {
+        chunks[i] = lp.bundles[i].nK; groups[i] = lp.bundles[i].gcnt;
+    }
+    return (int)lp.bundles.size();
+}
+
+// Feature-per-lane geometry of one level: grid size, 0 = take the other path, -1 = error.
+static int cb_fused_lane_geometry(CbFusedPlan* p, int level, int* slots_per_pass, int* smem_bytes, int* threads, int* chunks,
+                                  int* copies, int* bundle) {
+    const CbData& d = p->a.h.d;
+    const int grid = p->sm_count;                      // one block per SM
+    std::vector<int> gb(p->group_bins);
+    if (gb.empty()) gb.assign(d.G, p->a.h.B);
+    std::vector<float> share(p->group_share);
+    if (share.empty()) share.assign(d.G, 1.0f);
     cudaStream_t st = p->lane_stream;
-    cudaMemcpyAsync(p->d_btab[level], bundles.data(), bundles.size() * sizeof(CbBundle), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(p->d_items[level], items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(p->d_cap[level], cap.data(), cap.size() * sizeof(unsigned int), cudaMemcpyHostToDevice, st);
-    cb_lane_cap_kernel<<<grid, CB_LANE_THREADS, 256 * 32 * 4, st>>>(p->a.h.d, p->lanes, p->ldom, p->d_btab[level],
-                                                                    p->d_items[level], (int)items.size(), p->d_cap[level]);
-    if (cudaGetLastError() != cudaSuccess) return -1;
-    p->n_btab[level] = nbun;
-    p->n_items[level] = (int)items.size();
+    CbLanePlan lp;
+    for (int round = 0;; ++round) {
+        if (!cb_lane_plan(lp, d.n, d.G, gb.data(), share.data(), level, grid, p->lane_smem, p->a.h.work != nullptr, p->seq_docs)) return 0;
+        int occ = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cb_level_fused_kernel<true>, CB_LANE_THREADS, lp.smem) != cudaSuccess) { cudaGetLastError(); return -1; }
+        if (occ < 1) return 0;
+        const int nbun = (int)lp.bundles.size();
+        if (p->d_btab[level]) { cudaFree(p->d_btab[level]); p->d_btab[level] = nullptr; }
+        if (p->d_items[level]) { cudaFree(p->d_items[level]); p->d_items[level] = nullptr; }
+        if (p->d_cap[level]) { cudaFree(p->d_cap[level]); p->d_cap[level] = nullptr; }
+        if (cudaMalloc(&p->d_btab[level], (size_t)nbun * sizeof(CbBundle)) != cudaSuccess ||
+            cudaMalloc(&p->d_items[level], lp.items.size() * sizeof(int2)) != cudaSuccess ||
+            cudaMalloc(&p->d_cap[level], (size_t)nbun * sizeof(unsigned int)) != cudaSuccess) { cudaGetLastError(); return -1; }
+        cudaMemcpyAsync(p->d_btab[level], lp.bundles.data(), (size_t)nbun * sizeof(CbBundle), cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(p->d_items[level], lp.items.data(), lp.items.size() * sizeof(int2), cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(p->d_cap[level], lp.cap.data(), (size_t)nbun * sizeof(unsigned int), cudaMemcpyHostToDevice, st);
+        cb_lane_cap_kernel<<<grid, CB_LANE_THREADS, 256 * 32 * 4, st>>>(d, p->lanes, p->ldom, p->d_btab[level], p->d_items[level],
+                                                                        (int)lp.items.size(), p->d_cap[level]);
+        if (cudaGetLastError() != cudaSuccess) return -1;
+        // The shares come from a sample of the rows.  Where chunks are so large that a cell could receive more documents than
+        // it may, the count decides: too many in one bin, and the bundle is cut finer.
+        bool large = false, again = false;
+        for (int i = 0; i < nbun; ++i) large = large || lp.cap[i] > lp.limit[i] / 32;
+        if (!large || round == 3) break;
+        std::vector<unsigned int> got(nbun);
+        if (cudaMemcpyAsync(got.data(), p->d_cap[level], (size_t)nbun * sizeof(unsigned int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess) { cudaGetLastError(); return -1; }
+        for (int i = 0; i < nbun; ++i) {
+            if (got[i] <= lp.limit[i] + lp.limit[i] / 8) continue;
+            const float seen = (float)((double)got[i] * lp.bundles[i].nK / (double)d.n);
+            for (int q = 0; q < lp.bundles[i].gcnt; ++q) {
+                float& s = share[lp.bundles[i].g0 + q];
+                if (seen > s) { s = seen; again = true; }
+            }
+        }
+        if (!again) break;
+    }
+    p->n_btab[level] = (int)lp.bundles.size();
+    p->n_items[level] = (int)lp.items.size();
     p->lane_level[level] = 1;
-    p->lane_priv[level] = priv;
-    p->lane_list[level] = list;
-    *slots_per_pass = bundles[0].spp;
-    *smem_bytes = smem;
+    p->lane_priv[level] = lp.priv;
+    p->lane_list[level] = lp.list;
+    *slots_per_pass = lp.bundles[0].spp;
+    *smem_bytes = lp.smem;
     *threads = CB_LANE_THREADS;
-    *chunks = best;
+    *chunks = lp.chunks;
     *copies = 1;
-    *bundle = bundles[0].gcnt;
+    *bundle = lp.bundles[0].gcnt;
     return grid;
 }
 

@@ -47,7 +47,7 @@ __host__ __device__ __forceinline__ int cb_lane_extra_ints(int slots) {
 }
 
 // Largest fixed-point value.  From level 1 on it stays a few quanta below 2^23: a ring entry holds 24 bits, and the largest
-// value times its scale may round up.
+// value times its scale may round up.  (A cell of level 0 can receive 53 documents or more: the limit there never acts.)
 __device__ __forceinline__ float cb_lane_qmax(unsigned int cap, int level) {
     return fminf(level == 0 ? 1.0e9f : 8388600.0f, floorf(2147483647.0f / (float)(cap + 1u)) - 1.0f);
 }

@@ -274,6 +274,8 @@ class GpuObliviousEngine:
             self.lane_store = torch.empty(max(words, 1), dtype=torch.int32, device=self.dev)
             native.cuda_check(self.lib.cb_lane_store(ctypes.c_void_p(self.store.handle), _p(self.lane_store), self._stream()),
                               "cb_lane_store")
+            self.lib.cb_fused_set_lane_share(ctypes.c_void_p(self.plan), self.group_share.ctypes.data_as(ctypes.c_void_p),
+                                             int(len(self.group_share)))
             self.lib.cb_fused_set_lanes(ctypes.c_void_p(self.plan), _p(self.lane_store), _p(self.top_bins), self._stream())
         self.work = torch.zeros(self.store.G + 1, dtype=torch.int32, device=self.dev)
         if self.dynamic_work:
@@ -362,6 +364,8 @@ class GpuObliviousEngine:
         # every feature's most frequent bin (the feature-per-lane pass restores it from totals); -1 = padding column
         self.top_bins = torch.full((G * 4,), -1, dtype=torch.int16, device=self.dev)
         self.top_bins[: st.F] = 0
+        # per group, the largest share of the documents that one bin holds, those bins left out
+        self.group_share = np.ones(G, dtype=np.float32)
         if st.n <= 0 or st.F <= 0:
             return 0.0, None
         step = max(1, st.n // sample)
@@ -376,6 +380,9 @@ class GpuObliviousEngine:
             self.ctx.all_reduce_sum_(tot)
         top, arg = cnt.max(1)
         self.top_bins[: st.F] = arg[: st.F].to(torch.int16)
+        second = cnt.scatter(1, arg.unsqueeze(1), 0.0).amax(1) / tot.clamp_min(1.0)
+        second[st.F:] = 0.0
+        self.group_share = second.view(G, 4).amax(1).float().cpu().numpy()
         share = top / tot.clamp_min(1.0)
         mean_share = float(share[: st.F].mean().item())
         dom = torch.where(share >= 0.30, arg, torch.full_like(arg, 255))

@@ -212,3 +212,27 @@ def test_padding_columns_leave_the_scale_alone(F):
     assert _negative_mass_error(eng, store, y, n, (0, F - 1)) <= 0.5 * quantum / 1.0e-4 + 100 * 2.0 ** -20
     eng.finish()
     eng.close()
+
+
+def test_a_two_valued_column_leaves_the_scale_of_wide_tables_alone():
+    """Many columns leave few document chunks per row block; a column of two equally frequent values then fills a cell with a
+    quarter of a million documents.  The negatives' derivative (5e-4 of the positives') must not vanish in the steps."""
+    from catboost_b200.data.quantization import FlatFeature, make_store, pack_columns_into
+    n, F, p = 2_000_003, 600, 5.0e-4
+    widths = [2 if j % 32 == 7 else 129 for j in range(F)]
+    feats = [FlatFeature("float", j, borders=np.arange(w - 1, dtype=np.float32), n_bins=w) for j, w in enumerate(widths)]
+    store = make_store(feats, n, torch.device("cuda"))
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    for f0 in range(0, F, 64):
+        cols = torch.randint(0, 129, (min(64, F - f0), n), generator=gen, device="cuda", dtype=torch.uint8)
+        for j in range(len(cols)):
+            if widths[f0 + j] == 2:
+                cols[j] &= 1
+        pack_columns_into(store, cols, f0)
+    eng, y = _sure_engine(store, n, p=p)
+    eng.step(1)
+    torch.cuda.synchronize()
+    # at least 65534 steps to the largest derivative: half a step a negative, and fp32 sums of positives 20 times as heavy
+    assert _negative_mass_error(eng, store, y, n, (0, 7, 300, 583)) <= 0.5 / 65534 / p + 20 * 2.0 ** -20
+    eng.finish()
+    eng.close()
