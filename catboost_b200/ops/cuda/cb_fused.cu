@@ -337,7 +337,7 @@ struct CbFusedPlan {
     int lane_smem;                             // dynamic shared memory one block of that kernel may use
     int lane_level[CB_MAX_LEVELS];             // 1: the level takes that path
     long long lane_priv[CB_MAX_LEVELS];        // floats of its private tiles
-    long long lane_list[CB_MAX_LEVELS];        // entries of its document lists
+    int lane_list[CB_MAX_LEVELS];              // entries of a block's document list
     unsigned int* d_cap[CB_MAX_LEVELS];
 };
 
@@ -394,7 +394,7 @@ CB_API CbFusedPlan* cb_fused_create(const CbData* d, const CbComm* comm, unsigne
     if (cudaFuncGetAttributes(&fl, cb_level_fused_kernel<true>) != cudaSuccess) { cudaGetLastError(); delete p; return nullptr; }
     p->lane_smem = p->max_smem + (int)fa.sharedSizeBytes - (int)fl.sharedSizeBytes;
     for (int l = 0; l < CB_MAX_LEVELS; ++l) { p->lane_level[l] = 0; p->lane_priv[l] = 0; p->lane_list[l] = 0; p->d_cap[l] = nullptr; }
-    a.h.lanes = nullptr; a.h.ldom = nullptr; a.h.bcap = nullptr; a.h.list_q = nullptr; a.h.list_row = nullptr; a.h.nbundles = 0;
+    a.h.lanes = nullptr; a.h.ldom = nullptr; a.h.bcap = nullptr; a.h.list_q = nullptr; a.h.list_row = nullptr; a.h.list_len = 0; a.h.nbundles = 0;
     for (int l = 0; l < CB_MAX_LEVELS; ++l) { p->d_btab[l] = nullptr; p->d_items[l] = nullptr; p->d_gchunks[l] = nullptr; p->n_btab[l] = p->n_items[l] = 0; p->single_pass_bundle[l] = 0; }
     p->max_copies = 2;
     p->fuse_leaf_update = 1;
@@ -458,6 +458,7 @@ CB_API int cb_lane_store(const CbData* d, uint32_t* lanes, cudaStream_t st) {
     cb_lane_store_kernel<<<(int)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, st>>>(*d, lanes);
     return (int)cudaGetLastError();
 }
+// (lanes == nullptr: no level takes the path)
 CB_API void cb_fused_set_lanes(CbFusedPlan* p, const uint32_t* lanes, const short* ldom, cudaStream_t st) {
     p->lanes = lanes;
     p->ldom = ldom;
@@ -470,9 +471,9 @@ CB_API long long cb_fused_lane_priv(CbFusedPlan* p, int level) {
     return level < CB_MAX_LEVELS && p->lane_level[level] ? p->lane_priv[level] : 0;
 }
 
-// Document list entries (12 bytes each) of the level, and their place.
+// Document list entries (12 bytes each) of the level, all blocks, and their place.
 CB_API long long cb_fused_lane_list(CbFusedPlan* p, int level) {
-    return level < CB_MAX_LEVELS && p->lane_level[level] ? p->lane_list[level] : 0;
+    return level < CB_MAX_LEVELS && p->lane_level[level] ? (long long)p->lane_list[level] * p->sm_count : 0;
 }
 CB_API void cb_fused_set_lane_list(CbFusedPlan* p, int2* q, unsigned int* row) {
     p->a.h.list_q = q;
@@ -486,8 +487,8 @@ struct CbLanePlan {
     std::vector<int2> items;
     std::vector<unsigned int> cap;     // documents a lane total can receive
     std::vector<unsigned int> limit;   // documents a cell may receive
-    int smem = 0, chunks = 0;
-    long long priv = 0, list = 0;      // floats of private tiles, document list entries
+    int smem = 0, chunks = 0, list = 0;        // document list entries of a block
+    long long priv = 0;                // floats of private tiles
 };
 
 // Documents one cell may receive.  The fixed-point scale is 2^31 / (documents of the fullest cell), so this is the number of
@@ -505,6 +506,10 @@ static unsigned int cb_lane_cell_limit(long long tile_bytes) {
 // holds, the most frequent bin of every feature left out.  False: the level takes the other path.
 static bool cb_lane_plan(CbLanePlan& out, long long n, int G, const int* gb, const float* share, int level, int grid, int lane_smem,
                          bool counter, long long seq_docs) {
+    // One feature group leaves three quarters of a 32-byte sector unread (10.5M x 4: 0.90 against 0.78 ms an iteration on
+    // the other path; 10.5M x 8: 0.90 against 0.85, 1.2M x 8 even, 100K x 8 0.28 against 0.30, from 12 columns on faster).
+    // Document and row numbers are 32 bits wide, two work strides beyond the last document included.
+    if (level >= CB_MAX_LEVELS || n >= (1ll << 28) || !(G > 2 || (G == 2 && n < (1ll << 22)))) return false;
     const int nslots = level == 0 ? 1 : (1 << (level - 1));
     const int ints = lane_smem / 4 - cb_lane_extra_ints(0);
     std::vector<CbBundle>& bundles = out.bundles;
@@ -523,7 +528,7 @@ static bool cb_lane_plan(CbLanePlan& out, long long n, int G, const int* gb, con
         if (spp > nslots) spp = nslots;
         const int np = (nslots + spp - 1) / spp;
         spp = (nslots + np - 1) / np;
-        *b = CbBundle{g, gc, B, 1, spp, np, 1, FL, 0, 0, 0, 0, 0};
+        *b = CbBundle{g, gc, B, 1, spp, np, 1, FL, 0, 0, 0};
         return np * 25.0 + taken * (FL == 32 ? 3.2 : (FL == 16 ? 2.2 : 1.2));
     };
     for (int g = 0; g < G; g += 8) {
@@ -619,8 +624,8 @@ static bool cb_lane_plan(CbLanePlan& out, long long n, int G, const int* gb, con
     }
     int unit = 0;
     int& best = out.chunks;
-    long long &priv = out.priv, &list = out.list;
-    best = 1; priv = list = 0;
+    long long& priv = out.priv;
+    best = 1; priv = 0; out.list = 0;
     out.cap.resize(nbun);
     for (int i = 0; i < nbun; ++i) {
         CbBundle& b = bundles[i];
@@ -630,9 +635,9 @@ static bool cb_lane_plan(CbLanePlan& out, long long n, int G, const int* gb, con
         b.priv0 = priv;
         unit += nslots * (b.B >> 2) * NS;
         priv += (long long)b.nK * nslots * b.B * NS * 32;
-        b.list_stride = (int)((nblk + b.nK - 1) / b.nK) * (2 * CB_LANE_THREADS);
-        b.list0 = list;
-        if (b.seq && b.npass > 1) list += (long long)b.nK * b.list_stride;
+        // an item lists its documents for its own later passes, so a block needs room for one chunk
+        const int docs = (int)((nblk + b.nK - 1) / b.nK) * (2 * CB_LANE_THREADS);
+        if (b.seq && b.npass > 1 && docs > out.list) out.list = docs;
         // documents one lane total can receive
         out.cap[i] = (unsigned int)(((nblk + b.nK - 1) / b.nK) * (2 * CB_LANE_THREADS / 32) + 1);
     }
@@ -647,6 +652,28 @@ static bool cb_lane_plan(CbLanePlan& out, long long n, int G, const int* gb, con
             if (k < bundles[bi].nK)
                 for (int ps = 0; ps < per[bi]; ++ps) items.push_back(make_int2(bi | (ps << 16), k));
     return true;
+}
+
+// Device memory of the path for a tree of `depth` levels: the second copy of the store, the private tiles and the document
+// lists of the level with the most.  0: no level takes it.
+CB_API long long cb_lane_bytes(long long n, int G, const int* group_bins, const float* share, int depth, int grid, int lane_smem) {
+    long long priv = 0, list = 0;
+    bool any = false;
+    for (int level = 0; level < depth; ++level) {
+        CbLanePlan lp;
+        if (!cb_lane_plan(lp, n, G, group_bins, share, level, grid, lane_smem, true, CB_LANE_SEQ_DOCS)) continue;
+        any = true;
+        priv = lp.priv > priv ? lp.priv : priv;
+        list = lp.list > list ? lp.list : list;
+    }
+    return any ? 4 * (cb_lane_store_words(n, G) + priv) + 12 * list * grid : 0;
+}
+CB_API long long cb_fused_lane_bytes(CbFusedPlan* p, int depth) {
+    const CbData& d = p->a.h.d;
+    std::vector<int> gb(p->group_bins);
+    if (gb.empty()) gb.assign(d.G, p->a.h.B);
+    if (p->group_share.empty()) return 0;
+    return cb_lane_bytes(d.n, d.G, gb.data(), p->group_share.data(), depth, p->sm_count, p->lane_smem);
 }
 
 // The same from sizes alone: document chunks and feature groups of every bundle; returns their number (0: the level takes the
@@ -730,10 +757,7 @@ CB_API int cb_fused_geometry(CbFusedPlan* p, int level, int* slots_per_pass, int
     const long long n = p->a.h.d.n;
     if (level < CB_MAX_LEVELS) {
         p->lane_level[level] = 0;
-        // One feature group leaves three quarters of a 32-byte sector unread (10.5M x 4: 0.90 against 0.78 ms an iteration on
-        // the other path; 10.5M x 8: 0.90 against 0.85, 1.2M x 8 even, 100K x 8 0.28 against 0.30, from 12 columns on faster).
-        // document and row numbers of that path are 32 bits wide, two work strides beyond the last document included
-        if (p->lanes && narrow && n < (1ll << 28) && (G > 2 || (G == 2 && n < (1ll << 22)))) {
+        if (p->lanes && narrow) {
             const int grid = cb_fused_lane_geometry(p, level, slots_per_pass, smem_bytes, threads, chunks, copies, bundle);
             if (grid != 0) return grid > 0 ? grid : 0;
         }
@@ -952,6 +976,7 @@ CB_API int cb_fused_launch(CbFusedPlan* p, int level, float* hprev, float* hcur,
     const bool table = bundle > 0 && level < CB_MAX_LEVELS && p->d_btab[level] != nullptr;
     const bool lanes = level < CB_MAX_LEVELS && p->lane_level[level];
     a.h.lanes = lanes ? p->lanes : nullptr; a.h.ldom = p->ldom; a.h.bcap = lanes ? p->d_cap[level] : nullptr;
+    a.h.list_len = lanes ? p->lane_list[level] : 0;
     a.h.nbundles = table ? p->n_btab[level] : 0;
     a.h.btab = table ? p->d_btab[level] : nullptr;
     a.h.bitems = table ? p->d_items[level] : nullptr;

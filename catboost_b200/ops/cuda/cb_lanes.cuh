@@ -209,8 +209,8 @@ static __device__ __forceinline__ void cb_lane_accumulate(const CbHistArgs& a, i
         }
     };
     // The list of the documents that later passes of this item take: entries as in the ring, with the slot of the level.
-    int2* lq = a.list_q + bd.list0 + (long long)chunk * bd.list_stride;
-    unsigned int* lr = a.list_row + bd.list0 + (long long)chunk * bd.list_stride;
+    int2* lq = a.list_q + (long long)blockIdx.x * a.list_len;
+    unsigned int* lr = a.list_row + (long long)blockIdx.x * a.list_len;
     if (bd.seq && slot_begin > 0) {
         const int cnt = *list_count;
         int i = warp * 32 + lane;

@@ -49,8 +49,6 @@ struct CbBundle {
     int unit0;
     long long priv0;
     int seq;           // 1: a work item takes its chunk through all slot passes, 0: every pass is an item of its own
-    int list_stride;   // seq: documents of a chunk at most, and where the bundle's lists start
-    long long list0;
 };
 
 struct CbHistArgs {
@@ -111,8 +109,9 @@ struct CbHistArgs {
     const uint32_t* lanes;
     const short* ldom;
     const unsigned int* bcap;
-    int2* list_q;               // scratch: documents that the later slot passes of a work item take
+    int2* list_q;               // scratch: documents that the later slot passes of a work item take, list_len for each block
     unsigned int* list_row;
+    int list_len;
     int nbundles;
     const CbSplit* prev_splits;
     const int* prev_iter;

@@ -268,18 +268,38 @@ class GpuObliviousEngine:
             self.domw = None
             if self.dominant_bin_share > gate:
                 self.lib.cb_fused_set_max_copies(ctypes.c_void_p(self.plan), 8)
+        self.work = torch.zeros(self.store.G + 1, dtype=torch.int32, device=self.dev)
+        if self.dynamic_work:
+            self.lib.cb_fused_set_work(ctypes.c_void_p(self.plan), _p(self.work))
+        self.lane_store = self.lane_list = None
         if self.lane_hist:
-            # the feature-per-lane histogram pass reads its own copy of the store: a document's 32 features side by side
+            self.lib.cb_fused_set_lane_share(ctypes.c_void_p(self.plan), self.group_share.ctypes.data_as(ctypes.c_void_p),
+                                             int(len(self.group_share)))
+            # its copy of the store and its scratch may take half of the memory that is left: evaluation sets, snapshots and
+            # other programs come after it.  (Ranks may decide differently: both passes leave the same histograms.)
+            need = int(self.lib.cb_fused_lane_bytes(ctypes.c_void_p(self.plan), self.depth))
+            left = (torch.cuda.mem_get_info(self.dev)[0] + torch.cuda.memory_reserved(self.dev)
+                    - torch.cuda.memory_allocated(self.dev))
+            self.lane_hist = 0 < need <= left // 2
+        try:
+            self._make_levels()
+        except torch.cuda.OutOfMemoryError:
+            if not self.lane_hist:
+                raise
+            self.lane_hist = False
+            self._make_levels()
+
+    def _make_levels(self):
+        """Launch geometry and scratch of every level, with the feature-per-bank histogram pass if ``lane_hist``."""
+        self.lane_store = self.lane_list = self.priv = None
+        if self.lane_hist:
+            # that pass reads its own copy of the store: a document's 32 features side by side
             words = int(self.lib.cb_lane_store_words(self.n, self.store.G))
             self.lane_store = torch.empty(max(words, 1), dtype=torch.int32, device=self.dev)
             native.cuda_check(self.lib.cb_lane_store(ctypes.c_void_p(self.store.handle), _p(self.lane_store), self._stream()),
                               "cb_lane_store")
-            self.lib.cb_fused_set_lane_share(ctypes.c_void_p(self.plan), self.group_share.ctypes.data_as(ctypes.c_void_p),
-                                             int(len(self.group_share)))
-            self.lib.cb_fused_set_lanes(ctypes.c_void_p(self.plan), _p(self.lane_store), _p(self.top_bins), self._stream())
-        self.work = torch.zeros(self.store.G + 1, dtype=torch.int32, device=self.dev)
-        if self.dynamic_work:
-            self.lib.cb_fused_set_work(ctypes.c_void_p(self.plan), _p(self.work))
+        self.lib.cb_fused_set_lanes(ctypes.c_void_p(self.plan), _p(self.lane_store), _p(self.top_bins), self._stream())
+        self.lib.cb_fused_set_priv(ctypes.c_void_p(self.plan), None, _p(self.statmax) if self.quantized_hist else None)
         self.level_geo = []
         for level in range(self.depth):
             spp, smem, thr, nk, cp, bd = (ctypes.c_int(0) for _ in range(6))

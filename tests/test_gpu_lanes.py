@@ -236,3 +236,34 @@ def test_a_two_valued_column_leaves_the_scale_of_wide_tables_alone():
     assert _negative_mass_error(eng, store, y, n, (0, 7, 300, 583)) <= 0.5 / 65534 / p + 20 * 2.0 ** -20
     eng.finish()
     eng.close()
+
+
+def test_tables_whose_second_copy_does_not_fit_take_the_other_pass(monkeypatch):
+    """The pass may take half of the free device memory; a fit that finds less grows its trees with the per-group pass."""
+    n, F = 30_011, 28
+    store, cols = _store(n, [129] * F, seed=2)
+    y = (cols[0] / 129.0 + 0.2 * np.random.default_rng(3).standard_normal(n)).astype(np.float32)
+    trees = []
+    for little in (False, True, None):
+        if little:
+            free = 2 * store.bins.numel() * 4            # room for the copy alone, not for the other half as well
+            monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (free, free))
+            monkeypatch.setattr(torch.cuda, "memory_reserved", torch.cuda.memory_allocated)      # nothing cached
+        else:
+            monkeypatch.undo()
+        eng = _engine(store, y, 6, little is not None)
+        assert eng.lane_hist == (little is False) and (eng.lane_store is not None) == (little is False)
+        eng.step(2)
+        trees.append(eng.finish())
+        eng.close()
+    assert np.array_equal(trees[1][0][0], trees[2][0][0])           # the first tree, bit for bit
+    assert np.array_equal(trees[0][0][0, :4, :2], trees[1][0][0, :4, :2])
+
+
+def test_no_second_copy_for_one_feature_group():
+    store, cols = _store(3_000, [129] * 4, seed=1)
+    eng = _engine(store, cols[0].astype(np.float32), 3, True)
+    assert eng.lane_store is None and not eng.lane_hist
+    eng.step(1)
+    eng.finish()
+    eng.close()

@@ -32,3 +32,24 @@ def test_no_cell_receives_so_many_documents_that_small_values_round_away(n, F, b
             fullest = max(share, 1.0 / 32.0) * n / chunks
             if chunks < min(blocks, 4096):
                 assert fullest <= (1 << (15 if level == 0 else 17)), (level, chunks, fullest)
+
+
+def _bytes(n, F, bins, depth, share=1.0 / 64):
+    from catboost_b200.ops import native
+    G = (F + 3) // 4
+    gb = np.full(G, (bins + 3) // 4 * 4, dtype=np.int32)
+    sh = np.full(G, share, dtype=np.float32)
+    P = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    return native.cuda_lib().cb_lane_bytes(n, G, P(gb), P(sh), depth, SMS, SMEM)
+
+
+@pytest.mark.parametrize("n,F", [(10_500_000, 28), (50_000_000, 1000), (20_000_000, 2000), (100_000_000, 800)])
+def test_device_memory_is_the_second_copy_and_little_else(n, F):
+    """Scratch is for the work items in flight: it must not grow with rows x row blocks (12 bytes each would be 19 GB at 50M x 1000)."""
+    copy = n * ((F + 3) // 4) * 4
+    assert copy <= _bytes(n, F, 129, 6) <= 1.15 * copy + (1 << 30)
+
+
+@pytest.mark.parametrize("n,F", [(10_500_000, 4), (10_500_000, 8), (1 << 28, 28)])
+def test_no_memory_for_a_pass_that_no_level_takes(n, F):
+    assert _bytes(n, F, 129, 6) == 0
