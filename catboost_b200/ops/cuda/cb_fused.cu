@@ -27,6 +27,9 @@
 #include <new>
 #include <vector>
 #include <algorithm>
+#include <functional>
+#include <queue>
+#include <utility>
 
 namespace cg = cooperative_groups;
 
@@ -310,7 +313,7 @@ __global__ void __launch_bounds__(LANES ? CB_LANE_THREADS : 1024, 1) cb_level_fu
 
 // ---- host side ---------------------------------------------------------------------------------------
 #define CB_MAX_LEVELS 16
-#define CB_LANE_SEQ_DOCS 23296                 // (14 steps of a thread block)
+#define CB_LANE_SEQ_DOCS 65536
 struct CbFusedPlan {
     CbFusedArgs a;
     int threads;
@@ -333,7 +336,7 @@ struct CbFusedPlan {
     const short* ldom;
     cudaStream_t lane_stream;                  // the stream the lane store was made on; the work lists go there too
     std::vector<float> group_share;            // see cb_lane_plan (empty: a bin may hold every document)
-    long long seq_docs;                        // documents per SM from which a work item takes its chunk through all slot passes
+    long long seq_docs;                        // documents of a chunk from which a work item takes it through all slot passes
     int lane_smem;                             // dynamic shared memory one block of that kernel may use
     int lane_level[CB_MAX_LEVELS];             // 1: the level takes that path
     long long lane_priv[CB_MAX_LEVELS];        // floats of its private tiles
@@ -464,6 +467,8 @@ CB_API void cb_fused_set_lanes(CbFusedPlan* p, const uint32_t* lanes, const shor
     p->ldom = ldom;
     p->lane_stream = st;
 }
+// Documents of a chunk from which a work item takes its chunk through all slot passes (call before cb_fused_geometry).
+CB_API void cb_fused_set_lane_seq(CbFusedPlan* p, long long docs) { p->seq_docs = docs; }
 // share[g]: see cb_lane_plan, host memory
 CB_API void cb_fused_set_lane_share(CbFusedPlan* p, const float* share, int G) { p->group_share.assign(share, share + G); }
 // Floats of private tiles the level needs when it takes the feature-per-lane path (0: it does not).
@@ -573,20 +578,26 @@ static bool cb_lane_plan(CbLanePlan& out, long long n, int G, const int* gb, con
     // thread block (and at most 4096, which keeps two strides inside 32 bits)
     const long long nblk = (n + 2 * CB_LANE_THREADS - 1) / (2 * CB_LANE_THREADS);
     const int most = (int)(nblk < 1 ? 1 : (nblk < 4096 ? nblk : 4096));
-    // A shard of many rows takes each chunk through all slot passes as one item: one scan, the other passes read its list, and
-    // blocks finish together although the leaves of two passes hold different numbers of documents.  A tile of 200 KB that
-    // every block zeroes, writes and has added up costs about 16 us, though, and the scan 0.7 ns a document and SM: below
-    // some 23K documents per SM the passes are items of their own, so that a block has one tile (400K x 39, 129 bins, level 7:
-    // 2.6 times the time with all passes in an item).
-    const bool many = n >= seq_docs * grid;
-    const int seq = many && nslots <= 256 ? 1 : 0;     // (a list entry has eight bits for the slot)
+    // An item takes its chunk through all slot passes (one scan, the other passes read its list), or every pass is an item of
+    // its own.  The former costs a tile a pass (200 KB that a block zeroes, writes and has added up: about 20 us), the latter a
+    // scan a pass (0.62 ns a document), and its items differ, because the leaves of two passes hold different numbers of
+    // documents (10.5M x 28: blocks finished between 98 and 230 us).  The line is at 64K documents a chunk.  An iteration, one
+    // item / items of their own: 4M x 28, 129 bins, depth 6 (27K) 0.72 / 0.64 ms; 4M x 100, 129 bins, depth 8 (54K) 2.96 /
+    // 2.83; 7M x 28, 129 bins, depth 6 (47K) 0.92 / 0.87; 10.5M x 28, 129 bins (71K) depth 6 1.14 / 1.13, depth 8 2.19 / 2.30;
+    // 7M x 100, 255 bins, depth 8 (95K) 5.52 / 6.90; 16M x 28, 255 bins, depth 8 (108K) 3.67 / 5.07.
+    bool mixed = false;
+    for (int i = 1; i < nbun; ++i) mixed = mixed || cost[i] != cost[0];
+    // items of different times are handed out by a counter in two rounds, where a second tile per block is small change
+    const int two = (mixed && counter) ? 2 : 1;
+    const int seq = n * nbun >= seq_docs * grid * two && nslots <= 256 ? 1 : 0;      // (a list entry has eight bits for the slot)
     double W = 0.0;
     long long min_items = 0;
-    bool mixed = false;
+    bool passes = false;
     std::vector<int> per(nbun), least(nbun);           // items a chunk of the bundle takes; fewest chunks
     for (int i = 0; i < nbun; ++i) {
         bundles[i].seq = seq;
         per[i] = seq ? 1 : bundles[i].npass;
+        passes = passes || per[i] > 1;
         W += cost[i];
         // chunks small enough that no cell receives more documents than it may (a lane total has a 32nd of them all)
         float sh = 1.0f / 32.0f;
@@ -596,31 +607,60 @@ static bool cb_lane_plan(CbLanePlan& out, long long n, int G, const int* gb, con
         least[i] = k < 1.0 ? 1 : (k > (double)most ? most : (int)k + 1);
         if (least[i] > most) least[i] = most;
         min_items += (long long)least[i] * per[i];
-        if (cost[i] != cost[0]) mixed = true;
     }
-    // items of different times are handed out by a counter in two rounds, where a second tile per block is small change
-    const int rounds = (mixed && counter && many) ? 2 : 1;
-    long long T = (long long)grid * rounds;
-    while (T < min_items) T += grid;
-    long long used = 0;
-    for (int i = 0; i < nbun; ++i) {
-        const double each = cost[i] / per[i];
-        int k = (int)((double)T * each / W);
-        k = k < least[i] ? least[i] : (k > most ? most : k);
-        bundles[i].nK = k;
-        used += (long long)k * per[i];
-    }
-    for (;;) {
-        int pick = -1;
-        double worst = 0.0;
+    // About `want` items, no bundle below its fewest chunks, evened out; returns the time (us) of the longest block.
+    auto cut = [&](long long want) {
+        long long used = 0;
         for (int i = 0; i < nbun; ++i) {
-            if (used + per[i] > T || bundles[i].nK >= most) continue;
-            const double t = cost[i] / per[i] / bundles[i].nK;
-            if (t > worst) { worst = t; pick = i; }
+            int k = (int)((double)want * cost[i] / per[i] / W);
+            k = k < least[i] ? least[i] : (k > most ? most : k);
+            bundles[i].nK = k;
+            used += (long long)k * per[i];
         }
-        if (pick < 0) break;
-        ++bundles[pick].nK;
-        used += per[pick];
+        for (;;) {
+            int pick = -1;
+            double worst = 0.0;
+            for (int i = 0; i < nbun; ++i) {
+                if (used + per[i] > want || bundles[i].nK >= most) continue;
+                const double t = cost[i] / per[i] / bundles[i].nK;
+                if (t > worst) { worst = t; pick = i; }
+            }
+            if (pick < 0) break;
+            ++bundles[pick].nK;
+            used += per[pick];
+        }
+        std::vector<std::pair<double, long long>> kinds;               // time of an item, items
+        for (int i = 0; i < nbun; ++i) {
+            const CbBundle& b = bundles[i];
+            kinds.push_back({2.5e-5 * (double)n / b.nK * cost[i] / per[i] + 3.0 + 8.0e-5 * b.spp * b.B * (b.FL == 32 ? 256 : 128),
+                             (long long)b.nK * per[i]});
+        }
+        std::sort(kinds.begin(), kinds.end(), std::greater<std::pair<double, long long>>());
+        std::priority_queue<double, std::vector<double>, std::greater<double>> blocks;
+        for (int i = 0; i < grid; ++i) blocks.push(0.0);
+        double last = 0.0;
+        for (const auto& kind : kinds)
+            for (long long i = 0; i < kind.second; ++i) {
+                const double t = blocks.top() + kind.first;
+                blocks.pop();
+                blocks.push(t);
+                last = t > last ? t : last;
+            }
+        return last;
+    };
+    long long T = (long long)grid * (seq ? two : 1);
+    while (T < min_items) T += grid;
+    double time = cut(T);
+    // Slot passes come in whole multiples: 86 passes of one bundle leave 62 SMs idle (1.2M x 28, 255 bins, level 9: 670 us).
+    // Cut finer where that fills the SMs better.
+    if (passes && counter && T == grid) {
+        long long finest = T;
+        for (long long t = 2 * T; t <= 4 * T; t += T) {
+            const double u = cut(t);
+            if (u < 0.9 * time) { time = u; finest = t; }
+        }
+        cut(finest);
+        T = finest;
     }
     int unit = 0;
     int& best = out.chunks;
@@ -646,7 +686,6 @@ static bool cb_lane_plan(CbLanePlan& out, long long n, int G, const int* gb, con
     for (int i = 0; i < nbun; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
         return cost[x] / per[x] / bundles[x].nK > cost[y] / per[y] / bundles[y].nK; });
-    items.reserve((size_t)used);
     for (int k = 0; k < best; ++k)
         for (int bi : order)
             if (k < bundles[bi].nK)

@@ -242,6 +242,7 @@ _SIGS = {
     "cb_lane_store": (c_int, [c_void_p, c_void_p, c_void_p]),
     "cb_fused_set_lanes": (None, [c_void_p, c_void_p, c_void_p, c_void_p]),
     "cb_fused_set_lane_share": (None, [c_void_p, c_void_p, c_int]),
+    "cb_fused_set_lane_seq": (None, [c_void_p, c_ll]),
     "cb_lane_bytes": (c_ll, [c_ll, c_int, c_void_p, c_void_p, c_int, c_int, c_int]),
     "cb_fused_lane_bytes": (c_ll, [c_void_p, c_int]),
     "cb_lane_plan_query": (c_int, [c_ll, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),

@@ -59,7 +59,7 @@ class GpuObliviousEngine:
                  der_fn=None, zero_mean_leaves: bool = False, max_bundle: int = 8,
                  fused_leaf_steps: bool = True, mvs_reg=None, leaf_backtracking: str = "AnyImprovement",
                  fuse_leaf_update: bool = True, dims: int = 1, skip_dominant_bin: bool = True,
-                 lane_hist: bool = False):
+                 lane_hist: bool = False, lane_seq_docs: Optional[int] = None):
         assert store.bins.is_cuda, "GpuObliviousEngine needs a CUDA store"
         if depth > 16:
             raise ValueError("depth must be <= 16")
@@ -150,6 +150,7 @@ class GpuObliviousEngine:
         self._check_each = os.environ.get("CB200_CHECK") == "1"      # invariants after every iteration (slow, debugging)
         self.skip_dominant_bin = bool(skip_dominant_bin) and os.environ.get("CB200_SKIP_DOMINANT", "1") != "0"
         self.lane_hist = bool(lane_hist) and self.narrow_hist and self.S == 2 and store.F > 0
+        self.lane_seq_docs = lane_seq_docs             # None: the geometry's own choice
         self.stats = torch.zeros((self.S, npad), dtype=f32, device=dev)
         self.scal = torch.zeros(4, dtype=f64, device=dev)
         self.iter_ptr = torch.zeros(1, dtype=i32, device=dev)
@@ -275,6 +276,8 @@ class GpuObliviousEngine:
         if self.lane_hist:
             self.lib.cb_fused_set_lane_share(ctypes.c_void_p(self.plan), self.group_share.ctypes.data_as(ctypes.c_void_p),
                                              int(len(self.group_share)))
+            if self.lane_seq_docs is not None:
+                self.lib.cb_fused_set_lane_seq(ctypes.c_void_p(self.plan), int(self.lane_seq_docs))
             # its copy of the store and its scratch may take half of the memory that is left: evaluation sets, snapshots and
             # other programs come after it.  (Ranks may decide differently: both passes leave the same histograms.)
             need = int(self.lib.cb_fused_lane_bytes(ctypes.c_void_p(self.plan), self.depth))

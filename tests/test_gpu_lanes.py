@@ -36,16 +36,17 @@ def _engine(store, y, depth, lane_hist, **kw):
     (1025, [129] * 9, 6, False),                     # three groups: 8 documents a load
     (30_011, [129] * 28, 6, False),                  # seven groups: 4 documents a load, several slot passes
     (30_011, [129] * 28, 6, True),
-    (260_003, [129] * 28, 6, False),                 # chunks for every SM: the later passes read the first one's list
+    (260_003, [129] * 28, 6, False),                 # a chunk for every SM
     (5_000, [256] * 18, 6, False),                   # the widest columns, a row block of five groups
     (20_007, [255] * 33 + [2] * 6, 7, False),        # a second row block of two groups
     (9_999, [129] * 13 + [16] * 25 + [2] * 40, 8, True),     # narrow columns next to wide ones
 ])
-def test_lane_histograms_equal_sums_in_64_bits(n, widths, depth, sparse):
+def test_lane_histograms_equal_sums_in_64_bits(n, widths, depth, sparse, lane_seq_docs=None):
     store, cols = _store(n, widths, seed=n + len(widths), sparse=sparse)
     rng = np.random.default_rng(n)
     y = (cols[0] / widths[0] + 0.3 * rng.standard_normal(n) + (cols[-1] > 0)).astype(np.float32)
-    eng = _engine(store, y, depth, True)
+    eng = _engine(store, y, depth, True, lane_seq_docs=lane_seq_docs)
+    assert (eng.lane_list is not None) == (lane_seq_docs == 0)
     eng.step(1)
     torch.cuda.synchronize()
     level = depth - 1
@@ -267,3 +268,21 @@ def test_no_second_copy_for_one_feature_group():
     eng.step(1)
     eng.finish()
     eng.close()
+
+
+@pytest.mark.parametrize("n,widths,depth,sparse", [
+    (1665, [129] * 12, 6, False),                    # two chunks, the second of one document
+    (5_000, [256] * 18, 6, False),                   # the widest columns
+    (260_003, [129] * 28, 6, False),                 # three slot passes, a chunk for every SM and a short last one
+    (100_003, [129] * 40 + [3] * 9, 7, True),        # bundles of different lane widths: two rounds from the counter
+    (20_007, [255] * 33 + [2] * 6, 8, False),        # many slot passes
+])
+def test_work_items_with_all_slot_passes_equal_sums_in_64_bits(n, widths, depth, sparse):
+    """Large tables: an item takes its chunk through all slot passes, the later ones read the list that the first one wrote."""
+    test_lane_histograms_equal_sums_in_64_bits(n, widths, depth, sparse, lane_seq_docs=0)
+
+
+@pytest.mark.parametrize("n", [1, 1663, 1665, 30_011])
+@pytest.mark.parametrize("F", [5, 9, 12, 28, 41])
+def test_level_0_equals_sums_in_64_bits(n, F):
+    test_lane_histograms_equal_sums_in_64_bits(n, [129] * F, 1, False)

@@ -53,3 +53,14 @@ def test_device_memory_is_the_second_copy_and_little_else(n, F):
 @pytest.mark.parametrize("n,F", [(10_500_000, 4), (10_500_000, 8), (1 << 28, 28)])
 def test_no_memory_for_a_pass_that_no_level_takes(n, F):
     assert _bytes(n, F, 129, 6) == 0
+
+
+@pytest.mark.parametrize("n,F,bins,level", [(1_200_000, 28, 256, 9), (1_200_000, 100, 256, 7), (4_000_000, 100, 256, 7)])
+def test_slot_passes_that_come_in_whole_multiples_leave_few_sms_idle(n, F, bins, level):
+    """86 passes of one bundle as 86 items would leave 62 of 148 SMs without work."""
+    items = 0
+    for chunks, groups in _plan(n, F, bins, 1.0 / bins, level):
+        lanes = 64 if groups > 4 else 32
+        slots = min((SMEM // 4 - 26 * 256) // (bins * lanes + 64), 1 << (level - 1))
+        items += chunks * -(-(1 << (level - 1)) // slots)
+    assert items / (-(-items // SMS) * SMS) >= 0.85, items
