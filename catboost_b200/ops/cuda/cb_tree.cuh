@@ -974,6 +974,12 @@ __device__ __forceinline__ unsigned int cb_score_tag(const CbScoreArgs& a) {
     return a.ll_epoch ? cb_ll_tag(*a.ll_epoch + 1ull) : 0u;
 }
 
+__device__ __forceinline__ float cb_score_src(const CbScoreArgs& a, int r, size_t idx, unsigned int tag) {
+    if (tag == 0u) return __ldcg(a.hsrc[r] + idx);
+    const unsigned long long* w = reinterpret_cast<const unsigned long long*>(a.hsrc[r]) + idx;
+    return __uint_as_float(cb_ll_load(w, tag, a.ll_timeout_ns, a.ll_status, CB_TIMEOUT_HIST_ARRIVE, r));
+}
+
 __device__ __forceinline__ void cb_score_add_leaf(int fn, float l2, float s, float w, float& num, float& den) {
     switch (fn) {
         default:
@@ -1173,6 +1179,62 @@ static __device__ void cb_score_accumulate(const CbScoreArgs& a, int f, int p0, 
     }
 }
 
+// The same for one leaf, one statistic and one bin after the other: few instructions.  At the first levels, where there are
+// warps for every leaf, fetching the code above takes longer than the trips to L2 that it saves when there are few of these:
+// few bins a lane, or few columns.  Score phase of levels 0 to 3, above / here: 3K x 12, 17 bins 11 to 13 / 8 to 9 us;
+// 4M x 12, 129 bins 17 to 20 / 12 to 15; 10.5M x 4 20 to 22 / 14 to 16; but 60K x 39, 255 bins 12 to 18 / 14 to 25.
+static __device__ void cb_score_accumulate_leaf(const CbScoreArgs& a, int f, int l, float* sc) {
+    const int lane = threadIdx.x & 31;
+    const int nb = a.d.feat_nb[f];
+    const int col0 = a.d.feat_off[f] - a.col_base;
+    const bool onehot = a.d.feat_onehot && a.d.feat_onehot[f];
+    const int V = (nb + 31) >> 5;
+    const unsigned int tag = cb_score_tag(a);
+    int p = 0;
+    bool computed = true;
+    if (a.level > 0) {
+        p = l & ((1 << (a.level - 1)) - 1);
+        computed = ((a.small_mask[p >> 5] >> (p & 31)) & 1u) == (unsigned int)l >> (a.level - 1);
+    }
+    float totw = 0.0f, exw = 0.0f;
+    for (int k = 0; k < 2 * 8; ++k) sc[k * 32 + lane] = 0.0f;
+#pragma unroll 1
+    for (int pass = 0; pass < a.S; ++pass) {           // weights first
+        const int st = pass == 0 ? a.S - 1 : pass - 1;
+        float* pre = sc + (pass == 0 ? 512 : 768) + lane;
+        const size_t base = ((size_t)p * a.S + st) * a.W + col0;
+        float run = 0.0f;
+        for (int k = 0; k < V; ++k) {
+            const int bin = lane * V + k;
+            float x = 0.0f;
+            if (bin < nb) {
+                for (int r = 0; r < a.nsrc; ++r) x += cb_score_src(a, r, base + bin, tag);
+                if (!computed) x = __ldcg(a.hprev + base + bin) - x;
+                if (a.hcur) a.hcur[((size_t)l * a.S + st) * a.W + col0 + bin] = x;
+            }
+            run += x;
+            pre[k * 32] = onehot ? x : run;
+        }
+        float inc = run;
+        for (int o = 1; o < 32; o <<= 1) {
+            const float t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        const float excl = onehot ? 0.0f : inc - run;
+        const float total = __shfl_sync(0xffffffffu, inc, 31);
+        if (pass == 0) { totw = total; exw = excl; continue; }
+#pragma unroll 1
+        for (int k = 0; k < V; ++k) {
+            const float slk = excl + pre[k * 32], wlk = exw + sc[512 + k * 32 + lane];
+            float n_ = sc[k * 32 + lane], d_ = sc[256 + k * 32 + lane];
+            cb_score_add_leaf(a.score_fn, a.l2, slk, fmaxf(wlk, 0.0f), n_, d_);
+            cb_score_add_leaf(a.score_fn, a.l2, total - slk, fmaxf(totw - wlk, 0.0f), n_, d_);
+            sc[k * 32 + lane] = n_;
+            sc[256 + k * 32 + lane] = d_;
+        }
+    }
+}
+
 // Best candidate of feature f from the num / den of its `parts` warps (CB_SCORE_WARP_FLOATS apart); this warp takes every
 // pstep-th row of 32 bins.  Borders are bins 0 .. nb-2 (one-hot: every value).
 static __device__ void cb_score_finalize(const CbScoreArgs& a, int f, const float* sc, int parts, int k0, float noise_std) {
@@ -1235,7 +1297,14 @@ static __device__ void cb_score_phase(const CbScoreArgs& a, int cta, int ncta, f
     if (wpc < 1 || nf <= 0) return;
     // warps per feature: the count with the fewest pairs in a row for a warp, over all rounds (a round costs about one more)
     int wpf = 1, fpc = wpc, best = 0x7fffffff;
-    for (int w = 1; w <= min(wpc, parents); w += (w + 1) >> 1) {
+    const int leaves = 1 << a.level;
+    // a warp for every leaf: see cb_score_accumulate_leaf
+    const bool single = leaves <= 8 && (nf <= 16 || a.d.TB <= 48 * a.d.F) && (long long)nf <= (long long)ncta * (wpc / leaves);
+    if (single) {
+        wpf = leaves;
+        fpc = (nf + ncta - 1) / ncta;
+    }
+    for (int w = 1; w <= min(wpc, parents) && !single; w = w < 4 ? w + 1 : (w & (w - 1) ? w / 3 * 4 : w / 2 * 3)) {      // 1 2 3 4 6 8 12 16 24
         const int fit = wpc / w, rounds = (nf + ncta * fit - 1) / (ncta * fit);
         const int cost = rounds * ((parents + w - 1) / w + 1);
         if (cost < best) { best = cost; wpf = w; fpc = min(fit, (nf + ncta * rounds - 1) / (ncta * rounds)); }
@@ -1245,7 +1314,8 @@ static __device__ void cb_score_phase(const CbScoreArgs& a, int cta, int ncta, f
     for (int fbase = a.f_begin + cta * fpc; fbase < a.f_end; fbase += ncta * fpc) {
         const int f = fbase + slot;
         const bool have = slot < fpc && f < a.f_end;
-        if (have) cb_score_accumulate(a, f, sub, wpf, sc);
+        if (have && single) cb_score_accumulate_leaf(a, f, sub, sc);
+        else if (have) cb_score_accumulate(a, f, sub, wpf, sc);
         if (ts) ts[1] = cb_globaltimer();
         if (wpf > 1) __syncthreads();
         __syncwarp();
