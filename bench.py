@@ -471,7 +471,7 @@ def main():
                                   bootstrap_param=float(o.bagging_temperature or 1.0), leaf_method=o.leaf_estimation_method,
                                   leaf_iterations=int(o.leaf_estimation_iterations), seed=0, ctx=ctx, reduce=reduce,
                                   leaf_backtracking=str(o.leaf_estimation_backtracking or "AnyImprovement"),
-                                  quantized_hist={"narrow": True, "wide": "wide", "float": False}[cells], lane_hist=True)
+                                  quantized_hist={"narrow": True, "wide": "wide", "float": False}[cells])
 
     def timed_run(cells, with_clocks):
         """K timed iterations (CUDA events around each, L2 flushed before each, max over ranks of the sum)."""

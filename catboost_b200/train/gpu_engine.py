@@ -59,7 +59,7 @@ class GpuObliviousEngine:
                  der_fn=None, zero_mean_leaves: bool = False, max_bundle: int = 8,
                  fused_leaf_steps: bool = True, mvs_reg=None, leaf_backtracking: str = "AnyImprovement",
                  fuse_leaf_update: bool = True, dims: int = 1, skip_dominant_bin: bool = True,
-                 lane_hist: bool = False, lane_seq_docs: Optional[int] = None):
+                 lane_hist: bool = True, lane_seq_docs: Optional[int] = None):
         assert store.bins.is_cuda, "GpuObliviousEngine needs a CUDA store"
         if depth > 16:
             raise ValueError("depth must be <= 16")

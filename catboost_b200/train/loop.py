@@ -696,7 +696,7 @@ def _run_fast(o, objective, store, eval_stores, y_train, w_train, base_train, ev
             reduce=("fused" if o.histogram_reduce in ("fused", None) else "nccl"), eval_sets=evs,
             quantized_hist={"narrow": True, "wide": "wide", "float": False}[o.histogram_cells or "narrow"],
             leaf_backtracking=str(o.leaf_estimation_backtracking or "AnyImprovement"), dims=K,
-            der_fn=der_fn, zero_mean_leaves=bool(der_fn is not None and getattr(objective, "zero_mean_leaves", False)), lane_hist=True)
+            der_fn=der_fn, zero_mean_leaves=bool(der_fn is not None and getattr(objective, "zero_mean_leaves", False)))
     phase_timing = os.environ.get("CB200_PHASE_TIMING") == "1" and getattr(eng, "plan", None)
     if phase_timing:
         eng.enable_phase_timing()       # developer aid: per-level phase times of the last tree go to stderr

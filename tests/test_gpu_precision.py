@@ -77,7 +77,7 @@ def test_fixed_point_tiles_equal_an_integer_oracle():
     n, F, B = 200_003, 12, 32
     X, y = _data(n, F, seed=3)
     store = _store_of(X, y, B)
-    eng = _engine(store, y, "narrow", 1, 2)
+    eng = _engine(store, y, "narrow", 1, 2, lane_hist=False)
     eng.step(1)
     torch.cuda.synchronize()
     grid, spp, smem, thr, nK, C, gpc = eng.level_geo[0]
@@ -122,7 +122,7 @@ def test_fused_leaf_update_equals_separate_pass():
     outs = []
     for fuse in (True, False):
         eng = _engine(store, y, "narrow", 6, 4, fuse_leaf_update=fuse, leaf_iterations=2, random_strength=1.0,
-                      bootstrap_type="Bayesian")
+                      bootstrap_type="Bayesian", lane_hist=False)
         eng.step(4)
         sp, vals, wts = eng.finish()
         outs.append((sp.copy(), vals.copy(), wts.copy(), eng.approx[:n].cpu().numpy()))
@@ -400,7 +400,8 @@ def test_dominant_bin_skipping_gives_the_same_trees():
     store = _store_of(X, y, 64)
     outs = []
     for skip in (True, False):
-        eng = _engine(store, y, "narrow", 6, 5, skip_dominant_bin=skip, leaf_iterations=2, random_strength=0.0)
+        eng = _engine(store, y, "narrow", 6, 5, skip_dominant_bin=skip, leaf_iterations=2, random_strength=0.0,
+                      lane_hist=False)
         assert (eng.domw is not None) == skip
         eng.step(5)
         sp, vals, wts = eng.finish()
@@ -428,7 +429,7 @@ def test_bundles_sized_by_their_own_bins_give_the_same_model(monkeypatch):
     for uniform in (False, True):
         if uniform:
             monkeypatch.setenv("CB200_UNIFORM_BINS", "1")
-        eng = _engine(store, y, "narrow", 8, 6, leaf_iterations=2)
+        eng = _engine(store, y, "narrow", 8, 6, leaf_iterations=2, lane_hist=False)
         geos.append(list(eng.level_geo))
         eng.step(6)
         loss = eng.learn_loss_history().copy()
