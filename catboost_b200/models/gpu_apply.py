@@ -12,11 +12,28 @@ thread (the reference's GPU evaluator is single-device: catboost/libs/model/cuda
 from __future__ import annotations
 
 import ctypes
+import os
+import threading
 
 import numpy as np
 import torch
 
 from ..ops import native
+
+
+_COPY_THREADS = 8
+
+
+def _fill(dst: torch.Tensor, src: torch.Tensor):
+    """dst = src, contiguous rows of host memory, by several threads: one moves a third of what memory can.  The framework's own
+    threads, unless the process has set their number low (launchers of several ranks set OMP_NUM_THREADS=1; a CPU fit sets
+    its thread_count)."""
+    threads = min(_COPY_THREADS, os.cpu_count() or 1)
+    if torch.get_num_threads() >= threads or dst.numel() < (1 << 18):
+        dst.copy_(src)
+        return
+    native.cpu_lib().cbc_copy(ctypes.c_void_p(dst.data_ptr()), ctypes.c_void_p(src.data_ptr()),
+                              ctypes.c_longlong(4 * dst.numel()), ctypes.c_int(threads))
 
 
 class GpuPredictor:
@@ -84,7 +101,6 @@ class GpuPredictor:
         self.total_leaf_floats = int(np.asarray(p["vals"]).size)
         self.wide = None
         self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)     # set by a device wait that ran out of time
-        import os
         mode = os.environ.get("CB200_PREDICT_WIDE", "auto")
         want = mode == "1" or (mode == "auto" and 7 * self.U > self.S and self.U > 200)
         if want and self.S > 0 and self.lib.cb_predict_wide_fits(self.F_stage, self.S, self.T, self.dims, self.total_leaf_floats):
@@ -188,7 +204,7 @@ class GpuPredictor:
                 m = r1 - r0
                 drain(k)
                 if not src_pinned:
-                    stage[k][:m].copy_(xt[r0:r1])            # by all cores: one moves a third of what memory can
+                    _fill(stage[k][:m], xt[r0:r1])
                 h_src = xt[r0:r1] if src_pinned else stage[k][:m]
                 # a short last chunk uses the front of the buffers as a dense [dims, m] block
                 d_out = dout[k].view(-1)[: self.dims * m].view(self.dims, m)
@@ -225,7 +241,6 @@ class MultiGpuPredictor:
         self.T, self.dims = self.parts[0].T, self.parts[0].dims
 
     def predict(self, X: np.ndarray, chunk_rows: int = 0) -> np.ndarray:
-        import threading
         X = np.ascontiguousarray(X, dtype=np.float32)
         n = X.shape[0]
         res = np.empty((n, self.dims), dtype=np.float64)

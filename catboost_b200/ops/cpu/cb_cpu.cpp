@@ -639,3 +639,14 @@ CBC_API void cbc_interleave_f32(const float* const* cols, int F, long long n, fl
         }
     }
 }
+
+// dst = src by `threads` threads, whatever number the environment or an earlier call has set for the others.
+CBC_API void cbc_copy(void* dst, const void* src, long long bytes, int threads) {
+    if (threads < 1) threads = 1;
+    const long long piece = ((bytes + threads - 1) / threads + 4095) / 4096 * 4096;
+#pragma omp parallel for schedule(static) num_threads(threads)
+    for (int t = 0; t < threads; ++t) {
+        const long long b0 = std::min(bytes, t * piece), b1 = std::min(bytes, b0 + piece);
+        if (b1 > b0) std::memcpy(static_cast<char*>(dst) + b0, static_cast<const char*>(src) + b0, size_t(b1 - b0));
+    }
+}

@@ -127,6 +127,7 @@ def cpu_lib() -> ctypes.CDLL:
         lib.cbc_select_borders.restype = c_int
         lib.cbc_num_threads.restype = c_int
         lib.cbc_leaf_newton.restype = c_int
+        lib.cbc_copy.restype = None
         _cpu = lib
     return _cpu
 

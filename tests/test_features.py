@@ -1706,3 +1706,29 @@ def test_knn_search_on_the_host_is_exact():
     want = torch.topk(torch.cdist(Q, E), 6, dim=1, largest=False).indices
     assert torch.equal(got.sort(1).values, want.sort(1).values)
     assert ops.knn_search(Q, E[:3], 6).shape == (70, 3)                  # fewer cloud rows than k
+
+
+@pytest.mark.parametrize("shape", [(1, 1 << 18), (40_003, 9), (29_128, 9), (262_147, 1), (3, 7)])
+def test_apply_copies_rows_with_several_threads_whatever_the_process_allows(monkeypatch, shape):
+    """OMP_NUM_THREADS=1 (launchers of several ranks) or a CPU fit with thread_count=1 must not leave the rows to one core."""
+    import torch
+    from catboost_b200.models import gpu_apply
+    from catboost_b200.ops import native
+    lib, seen = native.cpu_lib(), []
+
+    class Lib:
+        @staticmethod
+        def cbc_copy(dst, src, size, threads):
+            seen.append(threads.value)
+            lib.cbc_copy(dst, src, size, threads)
+
+    monkeypatch.setattr(gpu_apply.native, "cpu_lib", lambda: Lib)
+    monkeypatch.setattr(gpu_apply.os, "cpu_count", lambda: 8)
+    src = torch.arange(shape[0] * shape[1], dtype=torch.float32).view(shape)
+    for threads in (1, 64):
+        monkeypatch.setattr(torch, "get_num_threads", lambda t=threads: t)
+        dst = torch.zeros(shape[0] + 1, shape[1])
+        seen.clear()
+        gpu_apply._fill(dst[:-1], src)
+        assert torch.equal(dst[:-1], src) and not dst[-1].any()
+        assert seen == ([8] if threads == 1 and src.numel() >= 1 << 18 else [])
