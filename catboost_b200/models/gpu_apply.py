@@ -152,9 +152,23 @@ class GpuPredictor:
                           "cb_predict_oblivious")
         return out
 
+    @staticmethod
+    def _chunk_rows(F: int, splits: int, parts: bool, pinned: bool) -> int:
+        """Rows of a staging buffer.  16 MB of floats, so that filling a buffer, its copy and its kernel overlap from 1M values
+        on (1M x 28 rows, 500 trees: 7.9 ms with one 256 MB buffer, 4.3 with these); page-locked rows, where nothing is
+        filled, go 256 MB at a time.  Buffers of few rows leave SMs idle, which a large model cannot hide behind the copy, so
+        a buffer grows with the splits to 64 MB (300K x 700, 1000 / 2000 / 6000 trees: 31 / 40 / 79 ms with 16 MB, 23 / 22 /
+        38 with 64 MB, 26 / 27 / 43 with 256 MB; 600K x 300, 2000 trees 31 / 24 / 31), and is 128 MB for a model that is
+        evaluated as a sum of tree ranges (100K x 2000, 2000 trees: 105 ms with 16 MB, 33 with 128 MB)."""
+        floats = 64 << 20
+        if not pinned:
+            floats = 32 << 20 if parts else min(16 << 20, max(4 << 20, 1400 * splits))
+        return max(4096, floats // max(F, 1))
+
     def predict(self, X: np.ndarray, chunk_rows: int = 0, out: np.ndarray = None) -> np.ndarray:
-        """Rows from host memory, in chunks through two pinned staging buffers and two streams: while one chunk is
-        copied to the device and evaluated, the host fills the other buffer, and results come back asynchronously."""
+        """Rows from host memory, in chunks through page-locked staging buffers, each with a stream (three above 64K rows, two
+        when the rows are page-locked already and go without staging): while one chunk is copied to the device and
+        evaluated, the host fills the next buffer, and results come back asynchronously."""
         X = np.ascontiguousarray(X, dtype=np.float32)
         n, F = X.shape
         res = np.empty((n, self.dims), dtype=np.float64) if out is None else out
@@ -163,11 +177,9 @@ class GpuPredictor:
         xt = torch.from_numpy(X)
         src_pinned = bool(xt.is_pinned())            # the caller's rows are page-locked: no staging copy needed
         if chunk_rows <= 0:
-            # 16 MB of floats per buffer, so that filling a buffer, its copy and its kernel overlap from 1M values on (1M x
-            # 28 rows, 500 trees: 7.9 ms with one 256 MB buffer); page-locked rows, where nothing is filled, go 256 MB at a
-            # time.  One geometry for every batch above 64K rows, so that the buffers kept from the previous call fit the
-            # next one whatever its length
-            chunk_rows = max(4096, ((64 if src_pinned else 4) << 20) // max(F, 1)) if n > 65536 else n
+            # one geometry for every batch above 64K rows, so that the buffers kept from the previous call fit the next one
+            # whatever its length
+            chunk_rows = self._chunk_rows(F, self.S, self.parts is not None, src_pinned) if n > 65536 else n
         with torch.cuda.device(self.dev):
             nbuf = (2 if src_pinned else 3) if n > 65536 else (2 if n > chunk_rows else 1)
             key = (chunk_rows, F, src_pinned, nbuf)
@@ -239,6 +251,19 @@ class MultiGpuPredictor:
         self.devices = [torch.device("cuda", int(d)) for d in devices]
         self.parts = [GpuPredictor(model, d) for d in self.devices]
         self.T, self.dims = self.parts[0].T, self.parts[0].dims
+
+    @staticmethod
+    def _chunk_rows(F: int, splits: int, parts: bool, pinned: bool) -> int:
+        """Rows of a staging buffer.  16 MB of floats, so that filling a buffer, its copy and its kernel overlap from 1M values
+        on (1M x 28 rows, 500 trees: 7.9 ms with one 256 MB buffer, 4.3 with these); page-locked rows, where nothing is
+        filled, go 256 MB at a time.  Buffers of few rows leave SMs idle, which a large model cannot hide behind the copy, so
+        a buffer grows with the splits to 64 MB (300K x 700, 1000 / 2000 / 6000 trees: 31 / 40 / 79 ms with 16 MB, 23 / 22 /
+        38 with 64 MB, 26 / 27 / 43 with 256 MB; 600K x 300, 2000 trees 31 / 24 / 31), and is 128 MB for a model that is
+        evaluated as a sum of tree ranges (100K x 2000, 2000 trees: 105 ms with 16 MB, 33 with 128 MB)."""
+        floats = 64 << 20
+        if not pinned:
+            floats = 32 << 20 if parts else min(16 << 20, max(4 << 20, 1400 * splits))
+        return max(4096, floats // max(F, 1))
 
     def predict(self, X: np.ndarray, chunk_rows: int = 0) -> np.ndarray:
         X = np.ascontiguousarray(X, dtype=np.float32)

@@ -1732,3 +1732,13 @@ def test_apply_copies_rows_with_several_threads_whatever_the_process_allows(monk
         gpu_apply._fill(dst[:-1], src)
         assert torch.equal(dst[:-1], src) and not dst[-1].any()
         assert seen == ([8] if threads == 1 and src.numel() >= 1 << 18 else [])
+
+
+def test_apply_buffers_grow_with_the_model():
+    from catboost_b200.models.gpu_apply import GpuPredictor
+    rows = GpuPredictor._chunk_rows
+    assert rows(28, 2_400, False, False) == (4 << 20) // 28                # copy and kernel overlap from 1M values on
+    assert rows(700, 36_000, False, False) == (16 << 20) // 700            # SMs idle with 6K rows
+    assert rows(2_000, 12_000, True, False) == (32 << 20) // 2_000
+    assert rows(28, 3_000, False, True) == (64 << 20) // 28
+    assert rows(100_000, 6, False, False) == 4_096
