@@ -48,6 +48,8 @@ class EvalSet:
 
 
 class GpuObliviousEngine:
+    LANE_BYTES_UNASKED = 512 << 20         # memory the feature-per-bank pass may take without a look at what is free
+
     def __init__(self, store: BinnedStore, target: torch.Tensor, weight: Optional[torch.Tensor], approx0: torch.Tensor,
                  objective, *, depth: int, iterations: int, learning_rate: float,
                  l2_leaf_reg: float, score_function: str = "Cosine", random_strength: float = 1.0,
@@ -280,10 +282,9 @@ class GpuObliviousEngine:
                 self.lib.cb_fused_set_lane_seq(ctypes.c_void_p(self.plan), int(self.lane_seq_docs))
             # its copy of the store and its scratch may take half of the memory that is left: evaluation sets, snapshots and
             # other programs come after it.  (Ranks may decide differently: both passes leave the same histograms.)
+            # Asking what is free takes 0.2 to 1.3 ms, so small tables just try.
             need = int(self.lib.cb_fused_lane_bytes(ctypes.c_void_p(self.plan), self.depth))
-            left = (torch.cuda.mem_get_info(self.dev)[0] + torch.cuda.memory_reserved(self.dev)
-                    - torch.cuda.memory_allocated(self.dev))
-            self.lane_hist = 0 < need <= left // 2
+            self.lane_hist = need > 0 and (need <= self.LANE_BYTES_UNASKED or 2 * need <= self._free_bytes())
         try:
             self._make_levels()
         except torch.cuda.OutOfMemoryError:
@@ -291,6 +292,11 @@ class GpuObliviousEngine:
                 raise
             self.lane_hist = False
             self._make_levels()
+
+    def _free_bytes(self) -> int:
+        """Device memory that this process can still get, the caching allocator's own included."""
+        return (torch.cuda.mem_get_info(self.dev)[0] + torch.cuda.memory_reserved(self.dev)
+                - torch.cuda.memory_allocated(self.dev))
 
     def _make_levels(self):
         """Launch geometry and scratch of every level, with the feature-per-bank histogram pass if ``lane_hist``."""

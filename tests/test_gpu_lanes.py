@@ -241,6 +241,7 @@ def test_a_two_valued_column_leaves_the_scale_of_wide_tables_alone():
 
 def test_tables_whose_second_copy_does_not_fit_take_the_other_pass(monkeypatch):
     """The pass may take half of the free device memory; a fit that finds less grows its trees with the per-group pass."""
+    from catboost_b200.train.gpu_engine import GpuObliviousEngine
     n, F = 30_011, 28
     store, cols = _store(n, [129] * F, seed=2)
     y = (cols[0] / 129.0 + 0.2 * np.random.default_rng(3).standard_normal(n)).astype(np.float32)
@@ -248,6 +249,7 @@ def test_tables_whose_second_copy_does_not_fit_take_the_other_pass(monkeypatch):
     for little in (False, True, None):
         if little:
             free = 2 * store.bins.numel() * 4            # room for the copy alone, not for the other half as well
+            monkeypatch.setattr(GpuObliviousEngine, "LANE_BYTES_UNASKED", 0)
             monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (free, free))
             monkeypatch.setattr(torch.cuda, "memory_reserved", torch.cuda.memory_allocated)      # nothing cached
         else:
@@ -286,3 +288,25 @@ def test_work_items_with_all_slot_passes_equal_sums_in_64_bits(n, widths, depth,
 @pytest.mark.parametrize("F", [5, 9, 12, 28, 41])
 def test_level_0_equals_sums_in_64_bits(n, F):
     test_lane_histograms_equal_sums_in_64_bits(n, [129] * F, 1, False)
+
+
+def test_allocation_failure_falls_back_to_the_other_pass(monkeypatch):
+    """Tables too small to ask for the free memory first: the allocation itself decides (made to fail on the host)."""
+    n, F = 3_001, 12
+    store, cols = _store(n, [129] * F, seed=2)
+    empty = torch.empty
+
+    def no_room(size, *a, **kw):
+        if size == words:
+            raise torch.cuda.OutOfMemoryError("out of memory")
+        return empty(size, *a, **kw)
+
+    from catboost_b200.ops import native
+    words = int(native.cuda_lib().cb_lane_store_words(n, 3))
+    monkeypatch.setattr(torch, "empty", no_room)
+    eng = _engine(store, cols[0].astype(np.float32), 4, True)
+    monkeypatch.undo()
+    assert not eng.lane_hist and eng.lane_store is None
+    eng.step(2)
+    assert (eng.finish()[0][:, :, 0] >= 0).any()
+    eng.close()
