@@ -440,9 +440,10 @@ __device__ __forceinline__ void cb_hist_q_apply(int* sh, int B, int C, int copy,
 //
 // NARROW: every cell is a single int32 (half of the atomics and of the tile).  The fixed-point scale is then limited by
 // the number of documents a cell can receive in this tile: qmax = (2^31 - 1) / (documents per chunk / replicas), about
-// 14 bits at 250K documents per chunk with two replicas.  Rounding is to nearest, so the error of a bin sum is an
-// unbiased random walk of at most half a quantum per document -- far below the sampling noise of the sum itself; the
-// leaf values never come from these histograms (the leaf pass re-accumulates exact derivatives).
+// 14 bits at 250K documents per chunk with two replicas.  Rounding is to nearest: for values of many quanta the error of a
+// bin sum is a random walk of at most half a quantum per document -- far below the sampling noise of the sum itself -- but
+// values below a few quanta all round the same way; the leaf values never come from these histograms (the leaf pass
+// re-accumulates exact derivatives).
 template <bool NARROW>
 static __device__ void cb_hist_item_q2(const CbHistArgs& a, int* sh, int g, long long item, int chunk, int nK,
                                        int slot_begin, int slot_count) {
@@ -1180,9 +1181,10 @@ static __device__ void cb_score_accumulate(const CbScoreArgs& a, int f, int p0, 
 }
 
 // The same for one leaf, one statistic and one bin after the other: few instructions.  At the first levels, where there are
-// warps for every leaf, fetching the code above takes longer than the trips to L2 that it saves when there are few of these:
-// few bins a lane, or few columns.  Score phase of levels 0 to 3, above / here: 3K x 12, 17 bins 11 to 13 / 8 to 9 us;
-// 4M x 12, 129 bins 17 to 20 / 12 to 15; 10.5M x 4 20 to 22 / 14 to 16; but 60K x 39, 255 bins 12 to 18 / 14 to 25.
+// warps for every leaf, fetching the code above takes longer than the trips to L2 that it saves when there are few of these --
+// few bins a lane -- or when a histogram phase of many rows has left none of it in the caches and columns are few.  Score
+// phase of levels 0 to 3, above / here: 3K x 12, 17 bins 11 to 13 / 8 to 9 us; 4M x 12, 129 bins 17 to 20 / 12 to 15;
+// 10.5M x 4 20 to 22 / 14 to 16; but 3K x 12, 129 bins 13 to 15 / 14 to 17, 60K x 39, 255 bins 12 to 18 / 14 to 25.
 static __device__ void cb_score_accumulate_leaf(const CbScoreArgs& a, int f, int l, float* sc) {
     const int lane = threadIdx.x & 31;
     const int nb = a.d.feat_nb[f];
@@ -1299,7 +1301,7 @@ static __device__ void cb_score_phase(const CbScoreArgs& a, int cta, int ncta, f
     int wpf = 1, fpc = wpc, best = 0x7fffffff;
     const int leaves = 1 << a.level;
     // a warp for every leaf: see cb_score_accumulate_leaf
-    const bool single = leaves <= 8 && (nf <= 16 || a.d.TB <= 48 * a.d.F) && (long long)nf <= (long long)ncta * (wpc / leaves);
+    const bool single = leaves <= 8 && (a.d.TB <= 48 * a.d.F || (nf <= 16 && a.d.n >= (1 << 20))) && (long long)nf <= (long long)ncta * (wpc / leaves);
     if (single) {
         wpf = leaves;
         fpc = (nf + ncta - 1) / ncta;

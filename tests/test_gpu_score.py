@@ -10,16 +10,16 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("widths,depth", [
     ([17] * 8, 1), ([17] * 8, 3), ([3] * 28, 4),                 # few bins: a warp for every leaf
-    ([129] * 12, 4), ([255] * 16, 2),                            # few columns: likewise
+    ([129] * 12, 4), ([255] * 16, 2),                            # few columns
     ([129] * 28, 4), ([129] * 28, 6), ([255] * 39, 8),           # pairs of children: 4, 16 and 64 of them
     ([256] * 3 + [2] * 30 + [65] * 7, 7),
 ])
-def test_best_split_has_the_best_score(widths, depth):
+def test_best_split_has_the_best_score(widths, depth, n=20_011):
     from catboost_b200.data.quantization import FlatFeature, make_store, pack_columns_into
     from catboost_b200.ops import native
     from catboost_b200.train.gpu_engine import GpuObliviousEngine
     from catboost_b200.train.objectives import make_objective
-    n, l2 = 20_011, 3.0
+    l2 = 3.0
     rng = np.random.default_rng(len(widths) + depth)
     cols = np.stack([rng.integers(0, w, n) for w in widths]).astype(np.uint8)
     feats = [FlatFeature("float", j, borders=np.arange(w - 1, dtype=np.float32), n_bins=w) for j, w in enumerate(widths)]
@@ -66,3 +66,9 @@ def test_best_split_has_the_best_score(widths, depth):
     assert score[f][col - int(off[f])] >= best * (1.0 - 1e-5)
     eng.finish()
     eng.close()
+
+
+@pytest.mark.parametrize("widths,depth", [([129] * 5, 2), ([255] * 16, 4)])
+def test_best_split_of_few_columns_and_many_rows(widths, depth):
+    """A warp for every leaf, whatever the number of bins, from 2^20 rows on."""
+    test_best_split_has_the_best_score(widths, depth, n=(1 << 20) + 7)
