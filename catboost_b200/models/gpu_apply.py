@@ -28,10 +28,10 @@ def _fill(dst: torch.Tensor, src: torch.Tensor):
     """dst = src, contiguous rows of host memory, by several threads: one moves a third of what memory can.  The framework's own
     threads, unless the process has set their number low (launchers of several ranks set OMP_NUM_THREADS=1; a CPU fit sets
     its thread_count)."""
-    threads = min(_COPY_THREADS, os.cpu_count() or 1)
-    if torch.get_num_threads() >= threads or dst.numel() < (1 << 18):
+    if dst.numel() < (1 << 18) or torch.get_num_threads() >= _COPY_THREADS:
         dst.copy_(src)
         return
+    threads = min(_COPY_THREADS, os.cpu_count() or 1)
     native.cpu_lib().cbc_copy(ctypes.c_void_p(dst.data_ptr()), ctypes.c_void_p(src.data_ptr()),
                               ctypes.c_longlong(4 * dst.numel()), ctypes.c_int(threads))
 
