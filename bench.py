@@ -616,7 +616,7 @@ def main():
         out = {"metric": "sec/1000 iters (device-timed, max over ranks)", "value": value, "unit": "s/1000iter",
                "n_gpus": world, "steps": K, "warmup": W, "ms_per_step": ms_per_step, "higher_is_better": False,
                "scaling": "strong", "vs_baseline": (value / base) if base else None,
-               "dtype": {"narrow": "fp32 statistics, histogram cells int32 fixed point (13-16 bit addends, exact integer sums)",
+               "dtype": {"narrow": "fp32 statistics, histogram cells int32 fixed point (addends of 14 to 23 bits, by the documents a cell can receive; exact integer sums)",
                          "wide": "fp32 statistics, histogram cells 24-bit fixed point in int32 hi/lo pairs (exact integer sums)",
                          "float": "fp32"}[args.cells],
                "data": "synthetic", "impl": "ours",

@@ -24,8 +24,9 @@
 #pragma once
 #include "cb_tree.cuh"
 
-// 26 warps: one block per SM, 72 registers a thread (the words of two batches stay in registers), and the staging areas leave
-// room for six slots of 32 features x 129 bins -- 16 slots, level 5, are three passes then and four with 28 warps.
+// 26 warps: one block per SM, 72 registers a thread (the words of two batches stay in registers; 34 words of the whole level
+// kernel are spilled), and the staging areas leave room for six slots of 32 features x 129 bins -- 16 slots, level 5, are
+// three passes then and four with 28 warps.
 #define CB_LANE_THREADS 832
 #define CB_LANE_RING 64                                // documents a warp's ring holds
 #define CB_LANE_STAGE_INTS (CB_LANE_RING * 3 + 64)     // {q0, q1 << 8 | slot} and the row number of each; 32 entries in flight

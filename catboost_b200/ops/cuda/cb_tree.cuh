@@ -1238,7 +1238,7 @@ static __device__ void cb_score_accumulate_leaf(const CbScoreArgs& a, int f, int
 }
 
 // Best candidate of feature f from the num / den of its `parts` warps (CB_SCORE_WARP_FLOATS apart); this warp takes every
-// pstep-th row of 32 bins.  Borders are bins 0 .. nb-2 (one-hot: every value).
+// `parts`-th row of 32 bins, from row k0 on.  Borders are bins 0 .. nb-2 (one-hot: every value).
 static __device__ void cb_score_finalize(const CbScoreArgs& a, int f, const float* sc, int parts, int k0, float noise_std) {
     const int lane = threadIdx.x & 31;
     const int nb = a.d.feat_nb[f];
